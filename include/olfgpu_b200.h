@@ -260,7 +260,8 @@ int olfgpu_last_fp64_refactors(int64_t context, unsigned char* flagged, int* cou
  * lane holding every LU block those levels produce (lanesPerTile then only sets the solves' narrow-level tiles; plans
  * whose narrow levels do not fit, and deferred-L plans, fall back to schedule 0); schedule 4 is schedule 3 with the
  * solves' narrow levels (the forward tail and the backward head) in shared memory as well, one CTA per lane holding
- * those rows' solution entries (lanesPerTile ignored); schedule -1 lets the next solve time every candidate on its
+ * those rows' solution entries (lanesPerTile ignored), or, from 512 buses on, the multifrontal form of the same block LU
+ * (one launch per level of its assembly tree; results within rounding); schedule -1 lets the next solve time every candidate on its
  * batch and keep the fastest (the autotuner).  olfgpu_get_schedule reports the schedule in force and, after an
  * autotuned solve, up to maxResults timings {schedule, lanesPerTile, threads, ms} into results (nResults receives
  * their count).

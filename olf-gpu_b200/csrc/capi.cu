@@ -254,7 +254,14 @@ extern "C" int olfgpu_structure_check_plan(int64_t structure, int plantedFault, 
         if (plantedFault < 0 || plantedFault > 3) throw std::runtime_error("plantedFault must be 0..3");
         if (!violations) throw std::runtime_error("null output");
         std::string first;
-        *violations = checkBlockPlan(structureOf(structure)->host.plan, plantedFault, first);
+        const Structure& s = structureOf(structure)->host;
+        const BlockPlan& plan = s.plan;
+        *violations = checkBlockPlan(plan, plantedFault, first);
+        if (plantedFault == 0 && !plan.deferredL) {   // the multifrontal form of the same factorization
+            const std::string mf = checkMfPlan(plan, s.nodeCol, buildMfPlan(plan, s.nodeCol));
+            if (!mf.empty()) ++*violations;
+            if (first.empty()) first = mf;
+        }
         if (firstViolation && capacity > 0) {
             const size_t k = std::min(first.size(), static_cast<size_t>(capacity - 1));
             std::memcpy(firstViolation, first.data(), k);

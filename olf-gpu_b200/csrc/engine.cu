@@ -719,6 +719,33 @@ std::shared_ptr<DeviceNet> uploadNet(const Structure& s) {
     d->fwdSplitD.upload(d->fwdSplit);
     d->bwdSplitD.upload(d->bwdSplit);
     buildSubtreeBins(*d, p, lrowLen, splitOf);
+    if (!p.deferredL && nb >= MF_MIN_BUSES) {
+        d->mf = buildMfPlan(p, s.nodeCol);
+        std::vector<MfNode> up, down;
+        std::vector<MfTask> task;
+        d->mfTaskPtr.assign(1, 0);
+        for (int l = 0; l < MF_LEAF_LEVELS && l + 1 < static_cast<int>(d->mf.upPtr.size()); l++) {
+            for (int x = d->mf.upPtr[l]; x < d->mf.upPtr[l + 1]; x++) {
+                const MfNode& n = d->mf.node[d->mf.upNode[x]];
+                const int rows = n.q <= MF_WARP_ROWS ? 1 : n.q;
+                for (int a = 0; a < rows; a++) {
+                    task.push_back(MfTask{n.q, rows > 1 ? a : -1, d->mf.rows[n.rows], n.rows, n.pan, n.trl, n.upd, n.u0});
+                }
+            }
+            d->mfTaskPtr.push_back(static_cast<int>(task.size()));
+        }
+        for (int t : d->mf.upNode) up.push_back(d->mf.node[t]);
+        for (int t : d->mf.downNode) down.push_back(d->mf.node[t]);
+        d->mfUp.upload(up);
+        d->mfDown.upload(down);
+        d->mfTask.upload(task);
+        d->mfRows.upload(d->mf.rows);
+        d->mfPan.upload(d->mf.pan);
+        d->mfTrl.upload(d->mf.trl);
+        d->mfRhs.upload(d->mf.rhs);
+        d->mfMore.upload(d->mf.more);
+        OLF_CUDA(prepareMf());
+    }
     d->coop = CoopPlan{static_cast<int>(p.levelPtr.size()) - 1, static_cast<int>(p.fwdLevelPtr.size()) - 1,
                        static_cast<int>(p.bwdLevelPtr.size()) - 1, d->levelPtrD.as<int>(), d->levelSplitD.as<int>(),
                        d->fwdPtrD.as<int>(), d->fwdPos.as<int>(), d->fwdSplitD.as<int>(), d->bwdPtrD.as<int>(),
@@ -772,6 +799,37 @@ std::shared_ptr<DeviceNet> uploadNet(const Structure& s) {
     // contexts' non-blocking streams would not wait for it
     OLF_CUDA(cudaDeviceSynchronize());
     return d;
+}
+
+std::shared_ptr<const MfSchedules> DeviceNet::mfSchedules(int nS, int share) const {
+    std::lock_guard<std::mutex> lock(mfMutex);
+    for (const auto& s : mfKept)
+        if (s->nS == nS && s->share == share) return s;
+    auto s = std::make_shared<MfSchedules>();
+    s->nS = nS;
+    s->share = share;
+    if (!mf.node.empty()) {
+        const int S = (nS + 31) / 32 * 32;
+        s->up64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, true);
+        s->up32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, true);
+        s->down64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, false);
+        s->down32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, false);
+    }
+    if (mfKept.size() >= 8) mfKept.erase(mfKept.begin());
+    mfKept.push_back(s);
+    return s;
+}
+
+MfRun DeviceNet::mfRun(const MfSchedules& s, void* updates) const {
+    MfRun r;
+    r.dev = MfDev{mfUp.as<MfNode>(), mfDown.as<MfNode>(), mfTask.as<MfTask>(), mfRows.as<int>(), mfPan.as<MfPanel>(),
+                  mfTrl.as<MfTrail>(), mfRhs.as<MfRhs>(), mfMore.as<int>(), std::max(mf.updBlocks, 1)};
+    r.up64 = &s.up64;
+    r.up32 = &s.up32;
+    r.down64 = &s.down64;
+    r.down32 = &s.down32;
+    r.upd = updates;
+    return r;
 }
 
 std::shared_ptr<DeviceNet> NetStructure::onDevice(int device) {
@@ -1163,8 +1221,32 @@ DevBatch fp64AllView(BatchContext& ctx) {
 
 }  // namespace
 
+// The launches and (on the first solve under schedule 4) the update matrices of the multifrontal solve; share: the
+// contexts of the graph launch, which run side by side.
+void prepareMultifrontal(BatchContext& ctx, int share) {
+    if (ctx.mfState == 2 || !ctx.regionFactor || !ctx.regionSolve || ctx.subtrees) return;
+    if (ctx.mfState == 1 && ctx.mfSchedules->share == share) return;
+    const DeviceNet& d = *ctx.dn;
+    const auto schedules = d.mfSchedules(ctx.nS, share);
+    if (ctx.mfState == 0) {
+        ctx.mfState = 2;
+        if (!schedules->fits()) return;
+        // one buffer for both precisions: a context's FP32 and FP64 factorizations never overlap
+        const size_t bytes = static_cast<size_t>(std::max(d.mf.updBlocks, 1)) * 4 * ctx.S * 8;
+        if (cudaMalloc(&ctx.mfUpd.p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            ctx.mfUpd.p = nullptr;
+            return;
+        }
+        ctx.mfUpd.bytes = bytes;
+        ctx.mfState = 1;
+    }
+    ctx.mfSchedules = schedules;
+    ctx.mfRun = d.mfRun(*schedules, ctx.mfUpd.p);
+}
+
 void captureIteration(BatchContext& ctx) {
-    const int key = ctx.narrowLanes * 100000 + (ctx.regionFactor ? 50000 : 0) + (ctx.regionSolve ? 20000 : 0) +
+    const int key = (ctx.multifrontal() ? 10000000 : 0) + ctx.narrowLanes * 100000 + (ctx.regionFactor ? 50000 : 0) + (ctx.regionSolve ? 20000 : 0) +
                     (ctx.subtrees ? 5000000 : 0) +
                     ctx.precision * 1000 +
                     ctx.refinementSteps * 10 +
@@ -1646,7 +1728,7 @@ cudaGraphConditionalHandle newHandle(cudaGraph_t owner) {
 // Appends one context's device-resident Newton loop to graph g as a branch with no dependencies: the loop state reset,
 // the WHILE node, the cap of lanes still iterating, and (withResults) the scenario-major result gather.  Three
 // capture streams: cs[0] for the branch, cs[1] for the WHILE body, cs[2] for the bodies nested in it.
-void appendNewtonLoop(BatchContext& ctx, cudaGraph_t g, const cudaStream_t* cs, bool withResults,
+void appendNewtonLoop(BatchContext& ctx, cudaGraph_t g, const cudaStream_t* cs, int share, bool withResults,
                       cudaEvent_t resultsDone) {
     const DeviceNet& dn = *ctx.dn;
     const DevNet& net = dn.view;
@@ -1655,6 +1737,7 @@ void appendNewtonLoop(BatchContext& ctx, cudaGraph_t g, const cudaStream_t* cs, 
     if (mixed && !ctx.lu32.p) ctx.lu32.alloc(static_cast<size_t>(net.nLu) * 4 * S * 4);
     if (!ctx.lu64.p) ctx.lu64.alloc(static_cast<size_t>(net.nLu) * 4 * S * 8);
     if (!ctx.loopState.p) ctx.loopState.alloc(8 * sizeof(int));
+    prepareMultifrontal(ctx, share);
     const DevBatch b = ctx.batch();
     const DevBatch b64 = fp64View(ctx), b64all = fp64AllView(ctx);
     DevBatch br = b;
@@ -1738,6 +1821,7 @@ void appendNewtonLoop(BatchContext& ctx, cudaGraph_t g, const cudaStream_t* cs, 
 long long loopKey(const BatchContext& ctx) {
     return ((((static_cast<long long>(ctx.narrowLanes) * 2 + (ctx.regionFactor ? 1 : 0)) * 2 + (ctx.regionSolve ? 1 : 0)) *
                  2 + (ctx.subtrees ? 1 : 0)) * 2 + ctx.precision) * 4096 * 64 +
+           (ctx.multifrontal() ? 1LL << 40 : 0) +
            static_cast<long long>(ctx.refinementSteps) * 4096 * 2 + ctx.mixedPolicy * 4096 + roundCap(ctx);
 }
 
@@ -1754,7 +1838,7 @@ int runDeviceLoop(BatchContext& ctx) {
         }
         cudaGraph_t g;
         OLF_CUDA(cudaGraphCreate(&g, 0));
-        appendNewtonLoop(ctx, g, ctx.loopStreams, false, nullptr);
+        appendNewtonLoop(ctx, g, ctx.loopStreams, 1, false, nullptr);
         OLF_CUDA(cudaGraphInstantiate(&ctx.loopGraph, g, 0));
         cudaGraphDestroy(g);
         ctx.loopGraphKey = key;
@@ -1778,6 +1862,7 @@ int runIterations(BatchContext& ctx) {
     const size_t S = ctx.S;
     if (mixed && !ctx.lu32.p) ctx.lu32.alloc(static_cast<size_t>(dn.view.nLu) * 4 * S * 4);
     if (!mixed && !ctx.lu64.p) ctx.lu64.alloc(static_cast<size_t>(dn.view.nLu) * 4 * S * 8);
+    prepareMultifrontal(ctx, 1);
     const int cap = roundCap(ctx);
     if (ctx.fallbackStart && ctx.hasX0Base && ctx.hasX0Full) selectStarts(ctx);
     if (ctx.deviceLoop && !ctx.phaseTiming && ctx.schedule != SCHEDULE_PERSISTENT && ctx.schedule != SCHEDULE_COOP) {
@@ -2180,7 +2265,7 @@ void launchMultiLoops(MultiContext& m) {
         m.loopCfgs.clear();
         for (size_t i = 0; i < k; i++) {
             BatchContext* c = m.members[i];
-            appendNewtonLoop(*c, g, m.capStreams, true, m.done[i]);
+            appendNewtonLoop(*c, g, m.capStreams, static_cast<int>(k), true, m.done[i]);
             m.loopKeys.push_back(loopKey(*c));
             m.loopBatches.push_back(c->batch());
             m.loopCfgs.push_back(c->cfg);

@@ -13,6 +13,7 @@
 #include "kernels.cuh"
 #include "coop.cuh"
 #include "persistent.cuh"
+#include "multifrontal.hpp"
 #include "structure.hpp"
 
 namespace olfb200 {
@@ -90,6 +91,15 @@ struct DeviceNet {
     std::vector<int> topLevelPtr, topLevelSplit, topFwdPtr, topFwdSplit, topBwdPtr, topBwdSplit, binPhasePtr,
         binFwdPhasePtr, binBwdPhasePtr;
     int binTasks = 0;               // LU blocks the bins factorize (of nLu)
+    // the multifrontal plan (no nodes: a deferred-L plan or a small grid) and its device tables
+    MfPlan mf;
+    std::vector<int> mfTaskPtr;      // the leaf levels' warp tasks
+    // the launches of a batch of nS lanes: planned on first use, the last few sizes kept
+    std::shared_ptr<const MfSchedules> mfSchedules(int nS, int share) const;
+    MfRun mfRun(const MfSchedules& s, void* updates) const;
+    mutable std::mutex mfMutex;
+    mutable std::vector<std::shared_ptr<const MfSchedules>> mfKept;
+    DeviceBuffer mfTask, mfRows, mfPan, mfTrl, mfRhs, mfMore, mfUp, mfDown;
 };
 
 // A structure and its device copies, one per device ordinal (uploaded on first use there).  Contexts hold their own
@@ -233,6 +243,14 @@ struct BatchContext {
     bool regionFactor = false;      // level schedule: the narrow factorization levels in shared memory
     bool regionSolve = false;       // level schedule: the solves' narrow levels in shared memory too
     bool subtrees = false;          // level schedule: the wide levels' independent subtrees as bins (schedule 5)
+    // schedule 4's linear solve: the multifrontal plan's launches for this batch and its update matrices.  Made on first
+    // use (prepareMultifrontal); mfState 2: a small grid, a panel that fits no CTA or no room on the device for the update
+    // matrices, and the level launches with their narrow levels in shared memory run instead
+    int mfState = 0;
+    std::shared_ptr<const MfSchedules> mfSchedules;
+    MfRun mfRun;
+    DeviceBuffer mfUpd;
+    bool multifrontal() const { return mfState == 1 && regionFactor && regionSolve && !subtrees; }
     Hybrid hybrid() const {
         const DeviceNet& d = *dn;
         Hybrid h{d.factorFrom, d.factorTo, d.fwdFrom, d.bwdUntil, narrowLanes, d.persistent};
@@ -253,6 +271,7 @@ struct BatchContext {
             h.uSlot = d.uSlot.as<int>();
             h.fwdRegionStart = d.fwdRegionStart.as<int>();
         }
+        if (multifrontal()) h.mf = &mfRun;
         return h;
     }
     bool useHybrid() const { return narrowLanes > 0 || regionFactor || regionSolve || subtrees; }

@@ -907,6 +907,10 @@ void launchSubtreeSolve(const DevNet& net, const DevBatch& b, const SubtreePlan&
 void launchFactor(const DevNet& net, const DevBatch& b, const int* levelPtr, const int* levelSplit, int nLevels,
                   bool fp32, const Hybrid* hybrid, cudaStream_t st) {
     clearTroubleKernel<<<(b.S + 127) / 128, 128, 0, st>>>(b);
+    if (hybrid && hybrid->mf) {
+        launchMfFactor(net, b, *hybrid->mf, fp32, st);
+        return;
+    }
     const bool region = hybrid && hybrid->regionSlots > 0;
     const bool range = hybrid && !region && hybrid->lanes > 0;
     const int wide = region ? hybrid->regionFrom : range ? hybrid->factorFrom : nLevels;
@@ -1191,6 +1195,10 @@ static void solveT(const DevNet& net, const DevBatch& b, T* w, const T* lu, cons
 
 void launchSolve(const DevNet& net, const DevBatch& b, const LevelSchedule& fwd, const LevelSchedule& bwd, bool fp32,
                  bool fromResidual, const Hybrid* hybrid, cudaStream_t st) {
+    if (hybrid && hybrid->mf && !fromResidual) {   // the forward solve of -F came with the factorization
+        launchMfBackward(net, b, *hybrid->mf, fp32, st);
+        return;
+    }
     if (fp32) solveT<float>(net, b, b.w32, b.lu32, fwd, bwd, fromResidual, hybrid, st);
     else solveT<double>(net, b, b.w64, b.lu64, fwd, bwd, fromResidual, hybrid, st);
 }

@@ -7,6 +7,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 namespace olfb200 {
 
 // Per-lane status codes (codes/gpu_ac_solver_status.cuh:10-15) and the engine's running state.
@@ -297,6 +299,63 @@ void launchSubtreeFactor(const DevNet& net, const DevBatch& b, const SubtreePlan
 void launchSubtreeSolve(const DevNet& net, const DevBatch& b, const SubtreePlan& sp, bool fp32, int dir,
                         cudaStream_t st);
 
+struct MfPlan;
+// The multifrontal linear solve (multifrontal.cu): the node tables, and per precision the launches of a context (one per
+// tree level; a launch's segments are its nodes by lanes per team).
+struct MfNode;
+struct MfTask;
+struct MfPanel;
+struct MfTrail;
+struct MfRhs;
+struct MfDev {
+    const MfNode* up;       // the nodes leaves first, level by level
+    const MfNode* down;     // the same nodes roots first, a level's small nodes before the others
+    const MfTask* task;     // the warps' tasks of the leaf levels
+    const int* rows;
+    const MfPanel* pan;
+    const MfTrail* trl;
+    const MfRhs* rhs;
+    const int* more;
+    int updBlocks;          // blocks of one lane's update matrices
+};
+struct MfSegment {
+    int first, count;     // nodes
+    int pairs, groups;    // lane pairs per CTA, groups of them in the batch
+};
+constexpr int MF_SEGMENTS = 6;                  // 16, 8, 4, 2 or 1 lane pairs per CTA
+constexpr int MF_SHARE_BYTES = 108 * 1024;      // a wide CTA's share of shared memory: two CTAs per SM
+constexpr int MF_MAX_BYTES = 112 * 1024;        // the largest panel's limit: two CTAs per SM
+struct MfLevel {
+    int taskFirst, taskCount;     // factorization: the warps' tasks of a leaf level; backward: the small nodes
+    int taskCtas, teamCtas;
+    int threads;                  // per CTA
+    int reverse;                  // lane groups of the tasks from the last to the first
+    int segments;
+    int smem;
+    MfSegment seg[MF_SEGMENTS];
+};
+struct MfSchedule {
+    std::vector<MfLevel> levels;
+};
+// A batch size's launches in both precisions (kept by the structure's device copy, DeviceNet::mfSchedules).
+struct MfSchedules {
+    int nS = 0, share = 1;
+    MfSchedule up64, up32, down64, down32;
+    bool fits() const { return !up64.levels.empty() && !up32.levels.empty() && !down64.levels.empty() && !down32.levels.empty(); }
+};
+struct MfRun {
+    MfDev dev{};
+    const MfSchedule *up64 = nullptr, *up32 = nullptr, *down64 = nullptr, *down32 = nullptr;
+    void* upd = nullptr;                                    // update matrices of every lane
+};
+// The launches of a batch of nS lanes (S with the padding) that runs beside share - 1 others; empty: some panel does not fit a CTA.
+MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int nS, int S, int share, bool fp32, bool factor);
+cudaError_t prepareMf();
+// Factorization and forward solve of -F (w holds y, the U blocks their storage; FP32 also the L blocks), and the backward
+// solve into dx.
+void launchMfFactor(const DevNet& net, const DevBatch& b, const MfRun& mf, bool fp32, cudaStream_t st);
+void launchMfBackward(const DevNet& net, const DevBatch& b, const MfRun& mf, bool fp32, cudaStream_t st);
+
 struct Hybrid {
     int factorFrom, factorTo, fwdFrom, bwdUntil, lanes;
     PersistentPlan plan;
@@ -312,6 +371,7 @@ struct Hybrid {
     const int* lrowSlot = nullptr;
     const int* uSlot = nullptr;
     const int* fwdRegionStart = nullptr;
+    const MfRun* mf = nullptr;           // the multifrontal solve in place of the level launches
 };
 // The shared-memory factorization of the narrow levels (two launches; no-op when h.regionSlots == 0; every region
 // level holds at most REGION_THREADS tasks).  prepareRegion raises the kernel's dynamic shared-memory limit for nSlots

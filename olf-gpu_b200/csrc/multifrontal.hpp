@@ -1,0 +1,85 @@
+// Host plan (multifrontal_plan.cpp) of the multifrontal block LU: the elimination order's columns grouped into nodes (supernodes)
+// that are factorized as small dense fronts, one tree level of nodes per launch (multifrontal.cu).
+#pragma once
+
+#include <string>
+#include <vector>
+
+#include "structure.hpp"
+
+namespace olfb200 {
+
+// A node eliminates the p pivots of its first p rows; its front has m = p + q rows (positions, ascending; the q others
+// belong to ancestors).  Its panel is the blocks U(k, j), k < p, j < m (index k m + j; for j < k the L part of the pivot
+// block) followed by L(i, k), p <= i < m (index p m + (i - p) p + k): p (m + q) blocks.  Its update matrix (the q x q
+// Schur complement it passes on, then q right-hand-side pairs, two to a block) starts at block upd of a buffer whose
+// slots are reused once the parent has read them.
+struct MfNode {
+    int p, q;
+    int rows;   // first of its m entries in rows / rhs
+    int pan;    // first of its panel records
+    int trl;    // first of its q q trailing records
+    int upd;    // first block of its update matrix
+    int child;  // 1: it has children (update matrices to add)
+    int u0;     // the LU block of its first pivot's diagonal (the rest of that U row follows)
+};
+
+// A warp's task near the leaves: a one-pivot node (row -1: all of it) or one row below its pivot.
+struct MfTask {
+    int q, row;
+    int pos;                       // the pivot's position
+    int rows, pan, trl, upd, u0;   // as its node's
+};
+
+// What a target adds up: s0 / s1 blocks of children's update matrices (-1 none); s1 <= -2: more[-2 - s1] = count,
+// then that many further blocks.
+struct MfPanel {
+    int aBlock;   // the Jacobian block, -1 none
+    int out;      // the LU block it ends in, -1 a structural zero of the pattern (not stored)
+    int s0, s1;
+};
+struct MfTrail {
+    int s0, s1;
+};
+// Right-hand side of one front row: the bus's two equation rows (their -F is added, pivot rows only; -1 else) and the
+// children's pairs (scalar index / 2 into the update buffer), encoded like the blocks.
+struct MfRhs {
+    int rowP, rowV;
+    int s0, s1;
+};
+
+struct MfPlan {
+    std::vector<MfNode> node;
+    std::vector<int> rows;              // positions of the front rows of every node
+    std::vector<MfPanel> pan;
+    std::vector<MfTrail> trl;
+    std::vector<MfRhs> rhs;
+    std::vector<int> more;
+    std::vector<int> parent;            // node -> parent node, -1 a root
+    // nodes by height above the leaves (factorization) and by depth below the roots (backward), within a level by panel
+    // size (backward: the small nodes first)
+    std::vector<int> upPtr, upNode, downPtr, downNode;
+    std::vector<int> downSmall;         // small nodes at the head of each backward level
+    int updBlocks = 0;                  // blocks of the update buffer (per lane)
+};
+
+// A node whose backward substitution one thread does per lane; the others get a CTA.
+inline bool mfSmall(const MfNode& n) { return n.p == 1 && n.q <= 8; }
+// Near the leaves (tree levels below MF_LEAF_LEVELS) every node has one pivot, and a warp factorizes it for 64 lanes (up
+// to MF_WARP_ROWS rows below the pivot; one row of it otherwise: four rows' blocks spill); further up a CTA does.
+// Factorization + solves per pass, 9,241 buses, 500 / 17 lanes, by leaf levels: 3 2.26 / 0.74 ms, 5 2.14 / 0.68 ms,
+// 7 2.13 / 0.68 ms, 9 2.09 / 0.69 ms; 2,000 buses, 257 lanes: 0.31, 0.33, 0.35, 0.36 ms.
+// Grids from here on take the multifrontal solve; below, the few levels of the level launches are the shorter chain (whole
+// solves, device time: 118 buses, 130 lanes 0.72 ms against 0.85 ms, 300 buses, 130 lanes 0.83 against 0.94, 1 lane 0.80
+// against 0.87; 2,000 buses, 1 / 16 / 257 lanes 0.84 / 1.19 / 2.55 ms against 0.62 / 0.84 / 2.03 ms).  The line depends on the
+// grid alone, so that a scenario's bits do not depend on its batch.
+constexpr int MF_MIN_BUSES = 512;
+constexpr int MF_MAX_PIVOTS = 16, MF_MAX_FRONT = 40, MF_LEAF_LEVELS = 5, MF_WARP_ROWS = 3;
+
+MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol);
+// "" when the plan holds: every position a pivot once, every LU block stored once, every Jacobian block and every
+// child's update block added exactly once and at its own row and column, children below their parents, and no update
+// matrix overwritten between its node's level and its parent's; else the first violation.
+std::string checkMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol, const MfPlan& m);
+
+}  // namespace olfb200
