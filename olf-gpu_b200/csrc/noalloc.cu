@@ -70,10 +70,10 @@ size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 // Byte offsets of the scratch regions for S lanes.
 struct ScratchLayout {
-    size_t J, lu, w, dx, F, active, pending, trouble, total;
+    size_t J, lu, w, dx, F, active, pending, trouble, total, upd, withUpd;
 };
 
-ScratchLayout layoutFor(const DevNet& net, size_t S, bool fp32) {
+ScratchLayout layoutFor(const DevNet& net, size_t updBlocks, size_t S, bool fp32) {
     ScratchLayout l{};
     size_t o = 0;
     l.J = o;
@@ -93,6 +93,9 @@ ScratchLayout layoutFor(const DevNet& net, size_t S, bool fp32) {
     l.trouble = o;
     o = align256(o + S * 4);
     l.total = o;
+    // the multifrontal solve's update matrices come last: a batch that fits without them only takes the level launches
+    l.upd = o;
+    l.withUpd = align256(o + updBlocks * 4 * S * (fp32 ? 4 : 8));
     return l;
 }
 
@@ -143,10 +146,11 @@ void linearSolveNoAlloc(const std::shared_ptr<NetStructure>& net, int nScenarios
     const DevNet& v = dn.view;
     const bool fp32 = precision == 1;
     const size_t S = static_cast<size_t>((nScenarios + 31) / 32 * 32);
-    const ScratchLayout lay = layoutFor(v, S, fp32);
+    const size_t updBlocks = std::max(dn.mf.updBlocks, 1);
+    const ScratchLayout lay = layoutFor(v, updBlocks, S, fp32);
     if (lay.total > NOALLOC_SCRATCH_BYTES) {
         size_t fit = 0;
-        for (size_t s2 = 32; layoutFor(v, s2, fp32).total <= NOALLOC_SCRATCH_BYTES; s2 += 32) fit = s2;
+        for (size_t s2 = 32; layoutFor(v, updBlocks, s2, fp32).total <= NOALLOC_SCRATCH_BYTES; s2 += 32) fit = s2;
         throw std::runtime_error("batch of " + std::to_string(nScenarios) + " scenarios needs " +
                                  std::to_string(lay.total) + " bytes of scratch; the no-allocation solve holds " +
                                  std::to_string(NOALLOC_SCRATCH_BYTES) + " bytes (at most " + std::to_string(fit) +
@@ -173,9 +177,20 @@ void linearSolveNoAlloc(const std::shared_ptr<NetStructure>& net, int nScenarios
     noallocInstallKernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(
         dn.csrToAD.as<int>(), csrVals, rhs, net->host.nnz, v.n, nScenarios, static_cast<int>(S), b.J, b.F, b.active,
         b.pending, b.trouble);
-    launchFactor(v, b, dn.levelPtr.data(), dn.levelSplit.data(), static_cast<int>(dn.levelPtr.size()) - 1, fp32,
-                 nullptr, st);
-    launchSolve(v, b, dn.fwd(), dn.bwd(), fp32, false, nullptr, st);
+    // FP64: the multifrontal solve where its update matrices fit the scratch (48 systems of the 2,000-bus grid: 26 dependent
+    // launches instead of 122), the level launches otherwise.  FP32 keeps the level launches: its rounding follows the
+    // summation order, and its results are those of the allocating entry point.
+    std::shared_ptr<const MfSchedules> mf;
+    if (!fp32 && lay.withUpd <= NOALLOC_SCRATCH_BYTES) mf = dn.mfSchedules(nScenarios, 1);
+    Hybrid hy{};
+    MfRun run;
+    if (mf && mf->fits()) {
+        run = dn.mfRun(*mf, base + lay.upd);
+        hy.mf = &run;
+    }
+    const Hybrid* hp = hy.mf ? &hy : nullptr;
+    launchFactor(v, b, dn.levelPtr.data(), dn.levelSplit.data(), static_cast<int>(dn.levelPtr.size()) - 1, fp32, hp, st);
+    launchSolve(v, b, dn.fwd(), dn.bwd(), fp32, false, hp, st);
     const size_t outCells = static_cast<size_t>(v.n) * nScenarios;
     noallocGatherKernel<<<(unsigned)((outCells + 255) / 256), 256, 0, st>>>(b.dx, b.trouble, out, v.n, nScenarios,
                                                                            static_cast<int>(S));
