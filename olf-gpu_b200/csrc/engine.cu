@@ -8,6 +8,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
+#include <system_error>
+#include <thread>
 
 namespace olfb200 {
 
@@ -845,6 +847,60 @@ std::shared_ptr<DeviceNet> NetStructure::find(int device) {
     std::lock_guard<std::mutex> lock(mu);
     auto it = devs.find(device);
     return it == devs.end() ? nullptr : it->second;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Results to host memory
+// ---------------------------------------------------------------------------------------------------------------
+HostReadback::~HostReadback() {
+    for (cudaEvent_t e : ready)
+        if (e) cudaEventDestroy(e);
+    if (ring) cudaFreeHost(ring);
+}
+
+bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    // (below four chunks the threads cost what they save)
+    if (pageable && bytes >= 4 * CHUNK && !ring) {
+        if (cudaMallocHost(&ring, SLOTS * CHUNK) != cudaSuccess) {
+            cudaGetLastError();
+            ring = nullptr;
+        }
+        for (cudaEvent_t& e : ready) OLF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    if (!pageable || bytes < 4 * CHUNK || !ring) {
+        OLF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+        return true;
+    }
+    const size_t chunks = (bytes + CHUNK - 1) / CHUNK;
+    cudaError_t err[SLOTS] = {};
+    auto work = [&](int slot, int slots) {
+        err[slot] = cudaSetDevice(device);
+        for (size_t c = slot; c < chunks && err[slot] == cudaSuccess; c += slots) {
+            const size_t at0 = c * CHUNK, len = std::min(CHUNK, bytes - at0);
+            unsigned char* pin = ring + static_cast<size_t>(slot) * CHUNK;
+            cudaError_t e = cudaMemcpyAsync(pin, static_cast<const unsigned char*>(src) + at0, len, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaEventRecord(ready[slot], st);
+            if (e == cudaSuccess) e = cudaEventSynchronize(ready[slot]);
+            if (e == cudaSuccess) std::memcpy(static_cast<unsigned char*>(dst) + at0, pin, len);
+            err[slot] = e;
+        }
+    };
+    const int slots = static_cast<int>(std::min<size_t>(chunks, std::min(SLOTS, std::max(1, static_cast<int>(std::thread::hardware_concurrency()) / 2))));
+    std::vector<std::thread> threads;
+    int mine = 0;     // slots whose thread could not be started run here
+    try {
+        for (int k = 1; k < slots; k++) threads.emplace_back(work, k, slots);
+    } catch (const std::system_error&) {
+        mine = static_cast<int>(threads.size()) + 1;
+    }
+    work(0, slots);
+    for (int k = mine; mine > 0 && k < slots; k++) work(k, slots);
+    for (std::thread& t : threads) t.join();
+    for (int k = 0; k < slots; k++) OLF_CUDA(err[k]);
+    return false;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -2177,9 +2233,7 @@ void solveBatch(BatchContext& ctx, const SolveRequest& req, double* out) {
     resultsKernel<<<grd, blk, 0, st>>>(ctx.x.as<double>(), ctx.iter.as<int>(), ctx.normOut.as<double>(),
                                        ctx.status.as<int>(), ctx.out.as<double>(), n, ctx.nS, ctx.S);
     OLF_CUDA(cudaEventRecord(e1, st));
-    if (out) {
-        OLF_CUDA(cudaMemcpyAsync(out, ctx.out.p, static_cast<size_t>(ctx.nS) * (n + 3) * 8, cudaMemcpyDeviceToHost, st));
-    }
+    if (out) ctx.readback.copy(ctx.device, out, ctx.out.p, static_cast<size_t>(ctx.nS) * (n + 3) * 8, st);
     OLF_CUDA(cudaStreamSynchronize(st));
     OLF_CUDA(cudaEventElapsedTime(&ctx.lastMs, e0, e1));
     cudaEventDestroy(e0);
@@ -2427,8 +2481,7 @@ void solveMulti(MultiContext& m, double* const* outs) {
                 cs = c.stream;
                 OLF_CUDA(cudaStreamWaitEvent(cs, m.done[i], 0));
             }
-            OLF_CUDA(cudaMemcpyAsync(outs[i], c.out.p, static_cast<size_t>(c.nS) * (c.net->host.n + 3) * 8,
-                                     cudaMemcpyDeviceToHost, cs));
+            m.readback.copy(m.device, outs[i], c.out.p, static_cast<size_t>(c.nS) * (c.net->host.n + 3) * 8, cs);
         }
     }
     OLF_CUDA(cudaStreamSynchronize(st));

@@ -57,6 +57,25 @@ struct DeviceBuffer {
     }
 };
 
+// Brings large results to pageable host memory through a small pinned ring, several threads copying out of it (and taking
+// the page faults of a fresh array) while the next chunks cross the bus.  Pinned or small destinations are copied directly.
+// 74 MB of results to a fresh array: 5 ms, against 26 ms for one pageable copy.
+class HostReadback {
+public:
+    HostReadback() = default;
+    HostReadback(const HostReadback&) = delete;
+    HostReadback& operator=(const HostReadback&) = delete;
+    ~HostReadback();
+    // Stream-ordered after what st holds; true: enqueued on st (the caller synchronises), false: the copy is complete.
+    bool copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st);
+
+private:
+    static constexpr size_t CHUNK = size_t(2) << 20;
+    static constexpr int SLOTS = 8;
+    unsigned char* ring = nullptr;      // pinned, SLOTS chunks, made on the first large copy
+    cudaEvent_t ready[SLOTS] = {};
+};
+
 // The structure's read-only device data (shared by every context built on it, on one device).
 struct DeviceNet {
     int device = 0;
@@ -277,6 +296,7 @@ struct BatchContext {
     bool useHybrid() const { return narrowLanes > 0 || regionFactor || regionSolve || subtrees; }
     std::vector<TuningResult> tuning;
     DeviceBuffer out;               // [nS][n + 3] scenario-major results
+    HostReadback readback;
     // reactive limits
     DevDs ds{};                     // distributed-slack participants (ds.nDs 0: none)
     DeviceBuffer dsRow, dsFactor, dsBase, dsMax, dsMin, dsPrev, dsFailed, dsRestartBuf;
@@ -382,6 +402,7 @@ struct MultiContext {
     cudaGraphExec_t graph = nullptr;
     int graphKey = -1;
     float lastMs = 0.f;
+    HostReadback readback;
     ~MultiContext();
 };
 

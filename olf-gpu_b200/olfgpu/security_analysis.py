@@ -99,10 +99,12 @@ class SecurityAnalysis:
                 dis = np.concatenate([dis, np.repeat(dis[:1], pad, axis=0)])
                 if xf is not None:
                     xf = np.concatenate([xf, np.repeat(xf[:1], pad, axis=0)])
+            # a full chunk's rows are written in place; a padded one's through an array of the chunk's width
             res = ctx.solve(x0, p.target, p.base_row_mode, dis, x0_full=xf, max_iter=max_iter, tol=tol,
                             reactive_limit_tol=reactive_limit_tol, max_outer=max_outer,
-                            max_pq_pv_switch=max_pq_pv_switch)
-            out[a:b] = res[: b - a]
+                            max_pq_pv_switch=max_pq_pv_switch, out=out[a:b] if b - a == width else None)
+            if b - a < width:
+                out[a:b] = res[: b - a]
             m, _, t = ctx.last_stats()
             tot[a:b] = t[: b - a]
             ms += m

@@ -1,0 +1,34 @@
+"""Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's threshold
+and its chunk size (2 MiB, from 8 MiB on)."""
+import numpy as np
+import pytest
+
+from conftest import grid
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("count", [1, 261, 262, 263, 328, 1049])
+def test_pageable_results_equal_pinned_ones(engine_lib, count):
+    import torch
+    from olfgpu import native, synthetic
+    g, p = grid("grid2000")
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    ctx = native.BatchContext(s, count)
+    ctx.set_schedule(native.LEVELS_SHARED_ALL, 0, 256)
+    dis = p.outage_masks(synthetic.draw_outages(g, count, seed=3))
+    pinned = torch.empty((count, p.n + 3), dtype=torch.float64).pin_memory().numpy()
+    ctx.solve(p.x_base, p.target, p.base_row_mode, dis, out=pinned)
+    fresh = ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
+    assert np.array_equal(fresh, pinned, equal_nan=True)
+
+
+def test_security_analysis_writes_chunks_in_place(engine_lib):
+    """A last chunk shorter than the others is padded and copied; every row equals the single batch's."""
+    from olfgpu import synthetic
+    from olfgpu.security_analysis import SecurityAnalysis
+    g, p = grid("grid118")
+    outs = synthetic.draw_outages(g, 50, seed=4)
+    sa = SecurityAnalysis(p)
+    whole, parts = sa.solve_n1(outs), sa.solve_n1(outs, chunk=16)
+    assert np.array_equal(whole.x, parts.x) and np.array_equal(whole.status, parts.status)
