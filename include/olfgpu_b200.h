@@ -485,7 +485,11 @@ int olfgpu_linear_solve_transposed(int64_t context, const double* csrVals, const
  *   copy_cols: dst[r, dstCol0 + c] (+)= src[r, srcCol0 + c], FP32.
  *   message_forward:  agg[b, i] = sum over directed edges e = (j -> i) not in sample b's outaged branch of
  *             relu(P[b, j] + Q[b, i] + C[e] + bmsg), PQ rows = [P | Q] (128 BF16), agg rows 64 BF16.
+ *   gemm_grad: Y = A . W [M x N]; accum [M x 64] += its first 64 columns (FP32, in place), second [M x (N - 64)] = the
+ *             rest (N = 128); with z and dz [M x 64]: dz = the new accum where z > 0, else 0, BF16.  Shapes (K, N): (64,128),
+ *             (128,64).
  *   message_backward: dPQ (FP32) and dC (FP32, summed over samples) of the same, by recomputation.
+ *   message_backward_bf16: the same with dPQ rounded to BF16.
  *   edge_project (C = Es . We) and its backward; relu_grad; adam (FP32 master weights, BF16 copy and transpose);
  *   mse (loss partials and its gradient).
  * olfgpu_gnn_last_error() reports the calling thread's last failure of these functions.
@@ -494,6 +498,8 @@ const char* olfgpu_gnn_last_error(void);
 int olfgpu_gnn_tc_timeouts(int* count);
 int olfgpu_gnn_gemm(int M, int K1, int K2, int N, const void* A1, const void* A2, const void* W, const float* bias,
                     int relu, const void* residual, void* outBf16, float* outF32, int ldo, void* saveZ, void* stream);
+int olfgpu_gnn_gemm_grad(int M, int K, int N, const void* A, const void* W, float* accum, float* second, const void* z,
+                         void* dz, void* stream);
 int olfgpu_gnn_gemm_dw(int M, int K1, int K2, int N, const void* A1, const void* A2, const void* dZ, float* dW,
                        float* db, float* partial, int maxChunks, void* stream);
 int olfgpu_gnn_message_forward(int B, int nb, const int* inPtr, const int* inEdge, const int* edgeSrc,
@@ -503,6 +509,10 @@ int olfgpu_gnn_message_backward(int B, int nb, int nEdges, const int* inPtr, con
                                 const int* outEdge, const int* edgeSrc, const int* edgeDst, const int* edgeBranch,
                                 const int* outage, const void* PQ, const float* C, const float* bmsg,
                                 const float* dAgg, float* dPQ, float* dC, void* stream);
+int olfgpu_gnn_message_backward_bf16(int B, int nb, int nEdges, const int* inPtr, const int* inEdge, const int* outPtr,
+                                const int* outEdge, const int* edgeSrc, const int* edgeDst, const int* edgeBranch,
+                                const int* outage, const void* PQ, const float* C, const float* bmsg,
+                                const float* dAgg, void* dPQ, float* dC, void* stream);
 int olfgpu_gnn_edge_project(int nEdges, const float* Es, const float* We, float* C, void* stream);
 int olfgpu_gnn_edge_project_backward(int nEdges, const float* Es, const float* dC, float* dWe, float* dbmsg,
                                      void* stream);

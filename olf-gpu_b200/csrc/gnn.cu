@@ -4,6 +4,7 @@
 // kernels for the messages.  Every reduction runs in a fixed order, so forward and backward are deterministic.
 //
 // Shapes: M rows = samples x buses; feature widths K, N are multiples of 16 / 8 (<= 128).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -98,13 +99,22 @@ __device__ __forceinline__ bool mbarWait(uint32_t mbar, uint32_t parity) {
     return false;
 }
 
-template <int K1, int K2, int N>
+// What a gradient GEMM does with its columns instead (GRAD): the first 64 are added to accum [M x 64] fp32 (in place), the
+// rest go to second [M x (N - 64)] fp32; with z, dz [M x 64] bf16 = the new accum where z > 0, else 0 (the next layer's ReLU).
+struct GradOut {
+    float* accum;
+    float* second;
+    const __nv_bfloat16* z;
+    __nv_bfloat16* dz;
+};
+
+template <int K1, int K2, int N, bool GRAD = false>
 __global__ void __launch_bounds__(128) gemmTcKernel(int M, const __nv_bfloat16* __restrict__ A1,
                                                     const __nv_bfloat16* __restrict__ A2,
                                                     const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                                                     int relu, const __nv_bfloat16* __restrict__ residual,
                                                     __nv_bfloat16* outB, float* outF, int ldo,
-                                                    __nv_bfloat16* saveZ) {
+                                                    __nv_bfloat16* saveZ, GradOut go = GradOut{}) {
     constexpr int K = K1 + K2;
     constexpr int KC = K / 8;                           // 16-byte chunks of a row
     constexpr int CL = KC < 4 ? KC : 4;                 // chunks of one row that a warp copies together
@@ -207,6 +217,50 @@ __global__ void __launch_bounds__(128) gemmTcKernel(int M, const __nv_bfloat16* 
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (r >= M) continue;
             float f[16];
+            if constexpr (GRAD) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) f[j] = __uint_as_float(v[j]);
+                if (cb >= 4) {
+                    constexpr int REST = N > 64 ? N - 64 : 0;
+                    float4* o = reinterpret_cast<float4*>(go.second + (size_t)r * REST + (cb - 4) * 16);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) o[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+                    continue;
+                }
+                const size_t at = (size_t)r * 64 + cb * 16;
+                float4* o = reinterpret_cast<float4*>(go.accum + at);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float4 a = o[j];
+                    a.x += f[4 * j];
+                    a.y += f[4 * j + 1];
+                    a.z += f[4 * j + 2];
+                    a.w += f[4 * j + 3];
+                    o[j] = a;
+                    f[4 * j] = a.x;
+                    f[4 * j + 1] = a.y;
+                    f[4 * j + 2] = a.z;
+                    f[4 * j + 3] = a.w;
+                }
+                if (go.dz) {
+                    const uint4* zp = reinterpret_cast<const uint4*>(go.z + at);
+                    const uint4 q[2] = {zp[0], zp[1]};
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t w4[4] = {q[h].x, q[h].y, q[h].z, q[h].w};
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const float2 zv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w4[j]));
+                            if (zv.x <= 0.f) f[h * 8 + 2 * j] = 0.f;
+                            if (zv.y <= 0.f) f[h * 8 + 2 * j + 1] = 0.f;
+                        }
+                    }
+                    uint4* d = reinterpret_cast<uint4*>(go.dz + at);
+                    d[0] = make_uint4(packBf2(f[0], f[1]), packBf2(f[2], f[3]), packBf2(f[4], f[5]), packBf2(f[6], f[7]));
+                    d[1] = make_uint4(packBf2(f[8], f[9]), packBf2(f[10], f[11]), packBf2(f[12], f[13]), packBf2(f[14], f[15]));
+                }
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 f[j] = __uint_as_float(v[j]) + sBias[cb * 16 + j];
@@ -255,10 +309,10 @@ __global__ void __launch_bounds__(128) gemmTcKernel(int M, const __nv_bfloat16* 
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-template <int K1, int K2, int N>
+template <int K1, int K2, int N, bool GRAD = false>
 void launchGemmTc(int M, const __nv_bfloat16* a1, const __nv_bfloat16* a2, const __nv_bfloat16* w, const float* bias,
                   int relu, const __nv_bfloat16* res, __nv_bfloat16* ob, float* of, int ldo, __nv_bfloat16* sz,
-                  cudaStream_t st) {
+                  cudaStream_t st, GradOut go = GradOut{}) {
     constexpr int smem = tcLaunchSmem(K1 + K2, N);
     // CTAs resident on the device: per SM the fewest that the shared memory (228 KB, 1 KB reserved per CTA), the
     // tensor memory (512 columns), the registers (64 K, 8-register granules) and the threads (2048) allow
@@ -266,13 +320,13 @@ void launchGemmTc(int M, const __nv_bfloat16* a1, const __nv_bfloat16* a2, const
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaFuncSetAttribute(gemmTcKernel<K1, K2, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+        if (cudaFuncSetAttribute(gemmTcKernel<K1, K2, N, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
                 cudaSuccess ||
-            cudaFuncSetAttribute(gemmTcKernel<K1, K2, N>, cudaFuncAttributePreferredSharedMemoryCarveout,
+            cudaFuncSetAttribute(gemmTcKernel<K1, K2, N, GRAD>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return -1;
         cudaFuncAttributes fa{};
-        if (cudaFuncGetAttributes(&fa, gemmTcKernel<K1, K2, N>) != cudaSuccess) return -1;
+        if (cudaFuncGetAttributes(&fa, gemmTcKernel<K1, K2, N, GRAD>) != cudaSuccess) return -1;
         const int regs = (fa.numRegs + 7) / 8 * 8;
         int perSm = 2048 / 128;
         perSm = std::min(perSm, 233472 / (smem + 1024));
@@ -285,11 +339,11 @@ void launchGemmTc(int M, const __nv_bfloat16* a1, const __nv_bfloat16* a2, const
     // 16-byte copies and stores: row pointers and the output stride must keep 16-byte alignment
     auto misaligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
     if (misaligned(a1) || (K2 > 0 && misaligned(a2)) || misaligned(res) || misaligned(ob) || misaligned(of) ||
-        misaligned(sz) || (ob && ldo % 8 != 0) || (of && ldo % 4 != 0) || ldo < N)
+        misaligned(sz) || misaligned(go.accum) || misaligned(go.second) || misaligned(go.z) || misaligned(go.dz) || (ob && ldo % 8 != 0) || (of && ldo % 4 != 0) || ldo < N)
         throw std::runtime_error("GEMM operands must be 16-byte aligned, ldo >= N and ldo * element size a multiple of 16");
     const long long tiles = (M + 127) / 128;
     const int grid = (int)(tiles < resident ? tiles : resident);
-    gemmTcKernel<K1, K2, N><<<grid, 128, smem, st>>>(M, a1, a2, w, bias, relu, res, ob, of, ldo, sz);
+    gemmTcKernel<K1, K2, N, GRAD><<<grid, 128, smem, st>>>(M, a1, a2, w, bias, relu, res, ob, of, ldo, sz, go);
 }
 
 // Partial weight gradients: chunk c of the rows contributes P_c[K x N] = [A1|A2]_c^T dZ_c and colsum(dZ_c); one CTA
@@ -406,14 +460,16 @@ __global__ void messageForwardKernel(int B, int nb, const int* inPtr, const int*
     float a0 = 0.f, a1 = 0.f;
     const int out = outage[b];
     const int p1 = inPtr[i + 1];
+#pragma unroll 4
     for (int p = inPtr[i]; p < p1; p++) {
         const int e = inEdge[p];
-        if (edgeBranch[e] == out) continue;
         const float2 pj = __bfloat1622float2(
             *reinterpret_cast<const __nv_bfloat162*>(PQ + ((size_t)b * nb + edgeSrc[e]) * 128 + f));
         const float2 c = *reinterpret_cast<const float2*>(C + (size_t)e * 64 + f);
-        a0 += fmaxf(pj.x + q0 + c.x, 0.f);
-        a1 += fmaxf(pj.y + q1 + c.y, 0.f);
+        if (edgeBranch[e] != out) {      // (the loads run either way, four edges' in flight)
+            a0 += fmaxf(pj.x + q0 + c.x, 0.f);
+            a1 += fmaxf(pj.y + q1 + c.y, 0.f);
+        }
     }
     *reinterpret_cast<__nv_bfloat162*>(agg + ((size_t)b * nb + i) * 64 + f) = __floats2bfloat162_rn(a0, a1);
 }
@@ -451,73 +507,90 @@ __global__ void messageForwardCompactKernel(int R, int nb, const int* rowNode, c
 }
 
 // Backward of the messages.  dQ[b, i] = sum over e into i of g_e; dP[b, j] = sum over e out of j of g_e, with
-// g_e = dAgg[b, dst(e)] * [pre_e > 0] recomputed from the saved P, Q.  Written into dPQ [rows x 128] (fp32).
-__global__ void messageBackwardNodesKernel(int B, int nb, const int* inPtr, const int* inEdge, const int* outPtr,
-                                           const int* outEdge, const int* edgeSrc, const int* edgeDst,
-                                           const int* edgeBranch, const int* outage, const __nv_bfloat16* PQ,
-                                           const float* C, const float* bmsg, const float* dAgg, float* dPQ) {
+// g_e = dAgg[b, dst(e)] * [pre_e > 0] recomputed from the saved P, Q.  Summed in fp32 and written into dPQ [rows x 128], as
+// fp32 or rounded to the bf16 that the next GEMMs read.  One warp per (sample, bus), a feature pair per lane: 4-byte and
+// 8-byte accesses (a warp reads whole 128 / 256-byte rows); bound by the gathers' latency.
+__device__ __forceinline__ float2 bf2(const __nv_bfloat16* p) {
+    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+}
+__device__ __forceinline__ void storePair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void storePair(__nv_bfloat16* p, float a, float b) {
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
+}
+
+template <typename OUT>
+__global__ void __launch_bounds__(256) messageBackwardNodesKernel(
+    int B, int nb, const int* __restrict__ inPtr, const int* __restrict__ inEdge, const int* __restrict__ outPtr,
+    const int* __restrict__ outEdge, const int* __restrict__ edgeSrc, const int* __restrict__ edgeDst,
+    const int* __restrict__ edgeBranch, const int* __restrict__ outage, const __nv_bfloat16* __restrict__ PQ,
+    const float* __restrict__ C, const float* __restrict__ bmsg, const float* __restrict__ dAgg, OUT* __restrict__ dPQ) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= B * nb) return;
     const int b = warp / nb, v = warp % nb;
     const int f = 2 * lane;
     const int out = outage[b];
-    const size_t rowV = (size_t)b * nb + v;
+    const size_t row0 = (size_t)b * nb, rowV = row0 + v;
+    const float2 bm = *reinterpret_cast<const float2*>(bmsg + f);
+    const float2 p = bf2(PQ + rowV * 128 + f), q = bf2(PQ + rowV * 128 + 64 + f);
     // as destination: dQ[v]
     {
-        const float q0 = __bfloat162float(PQ[rowV * 128 + 64 + f]) + bmsg[f];
-        const float q1 = __bfloat162float(PQ[rowV * 128 + 64 + f + 1]) + bmsg[f + 1];
-        const float d0 = dAgg[rowV * 64 + f], d1 = dAgg[rowV * 64 + f + 1];
+        const float q0 = q.x + bm.x, q1 = q.y + bm.y;
+        const float2 d = *reinterpret_cast<const float2*>(dAgg + rowV * 64 + f);
         float s0 = 0.f, s1 = 0.f;
-        for (int p = inPtr[v]; p < inPtr[v + 1]; p++) {
-            const int e = inEdge[p];
-            if (edgeBranch[e] == out) continue;
-            const size_t pj = ((size_t)b * nb + edgeSrc[e]) * 128 + f;
-            if (__bfloat162float(PQ[pj]) + q0 + C[(size_t)e * 64 + f] > 0.f) s0 += d0;
-            if (__bfloat162float(PQ[pj + 1]) + q1 + C[(size_t)e * 64 + f + 1] > 0.f) s1 += d1;
+        const int p1 = inPtr[v + 1];
+#pragma unroll 4
+        for (int x = inPtr[v]; x < p1; x++) {
+            const int e = inEdge[x];
+            const float2 pj = bf2(PQ + (row0 + edgeSrc[e]) * 128 + f);
+            const float2 c = *reinterpret_cast<const float2*>(C + (size_t)e * 64 + f);
+            const bool keep = edgeBranch[e] != out;
+            if (keep && pj.x + q0 + c.x > 0.f) s0 += d.x;
+            if (keep && pj.y + q1 + c.y > 0.f) s1 += d.y;
         }
-        dPQ[rowV * 128 + 64 + f] = s0;
-        dPQ[rowV * 128 + 64 + f + 1] = s1;
+        storePair(dPQ + rowV * 128 + 64 + f, s0, s1);
     }
     // as source: dP[v]
     {
-        const float p0 = __bfloat162float(PQ[rowV * 128 + f]), p1 = __bfloat162float(PQ[rowV * 128 + f + 1]);
         float s0 = 0.f, s1 = 0.f;
-        for (int p = outPtr[v]; p < outPtr[v + 1]; p++) {
-            const int e = outEdge[p];
-            if (edgeBranch[e] == out) continue;
-            const size_t rowI = (size_t)b * nb + edgeDst[e];
-            const float pre0 = p0 + __bfloat162float(PQ[rowI * 128 + 64 + f]) + bmsg[f] + C[(size_t)e * 64 + f];
-            const float pre1 = p1 + __bfloat162float(PQ[rowI * 128 + 64 + f + 1]) + bmsg[f + 1] + C[(size_t)e * 64 + f + 1];
-            if (pre0 > 0.f) s0 += dAgg[rowI * 64 + f];
-            if (pre1 > 0.f) s1 += dAgg[rowI * 64 + f + 1];
+        const int p1 = outPtr[v + 1];
+#pragma unroll 4
+        for (int x = outPtr[v]; x < p1; x++) {
+            const int e = outEdge[x];
+            const size_t rowI = row0 + edgeDst[e];
+            const float2 qi = bf2(PQ + rowI * 128 + 64 + f);
+            const float2 c = *reinterpret_cast<const float2*>(C + (size_t)e * 64 + f);
+            const float2 d = *reinterpret_cast<const float2*>(dAgg + rowI * 64 + f);
+            const bool keep = edgeBranch[e] != out;
+            if (keep && p.x + qi.x + bm.x + c.x > 0.f) s0 += d.x;
+            if (keep && p.y + qi.y + bm.y + c.y > 0.f) s1 += d.y;
         }
-        dPQ[rowV * 128 + f] = s0;
-        dPQ[rowV * 128 + f + 1] = s1;
+        storePair(dPQ + rowV * 128 + f, s0, s1);
     }
 }
 
 // dC[e] = sum over samples of g_e (one warp per directed edge, two features per lane); dbmsg from the partials of
 // dC summed over edges in edge order by the caller's reduction.
-__global__ void messageBackwardEdgesKernel(int B, int nb, int nEdges, const int* edgeSrc, const int* edgeDst,
-                                           const int* edgeBranch, const int* outage, const __nv_bfloat16* PQ,
-                                           const float* C, const float* bmsg, const float* dAgg, float* dC) {
+__global__ void __launch_bounds__(256) messageBackwardEdgesKernel(
+    int B, int nb, int nEdges, const int* __restrict__ edgeSrc, const int* __restrict__ edgeDst,
+    const int* __restrict__ edgeBranch, const int* __restrict__ outage, const __nv_bfloat16* __restrict__ PQ,
+    const float* __restrict__ C, const float* __restrict__ bmsg, const float* __restrict__ dAgg, float* __restrict__ dC) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= nEdges) return;
     const int e = warp, f = 2 * lane;
-    const int j = edgeSrc[e], i = edgeDst[e];
+    const int j = edgeSrc[e], i = edgeDst[e], branch = edgeBranch[e];
+    const float2 bm = *reinterpret_cast<const float2*>(bmsg + f);
+    const float2 c = *reinterpret_cast<const float2*>(C + (size_t)e * 64 + f);
     float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
     for (int b = 0; b < B; b++) {
-        if (edgeBranch[e] == outage[b]) continue;
-        const size_t rj = ((size_t)b * nb + j) * 128, ri = ((size_t)b * nb + i) * 128;
-        const float pre0 = __bfloat162float(PQ[rj + f]) + __bfloat162float(PQ[ri + 64 + f]) + bmsg[f] + C[(size_t)e * 64 + f];
-        const float pre1 = __bfloat162float(PQ[rj + f + 1]) + __bfloat162float(PQ[ri + 64 + f + 1]) + bmsg[f + 1] +
-                           C[(size_t)e * 64 + f + 1];
-        const size_t ai = ((size_t)b * nb + i) * 64 + f;
-        if (pre0 > 0.f) s0 += dAgg[ai];
-        if (pre1 > 0.f) s1 += dAgg[ai + 1];
+        const size_t rj = (size_t)b * nb + j, ri = (size_t)b * nb + i;
+        const float2 pj = bf2(PQ + rj * 128 + f), qi = bf2(PQ + ri * 128 + 64 + f);
+        const float2 d = *reinterpret_cast<const float2*>(dAgg + ri * 64 + f);
+        const bool keep = branch != outage[b];
+        if (keep && pj.x + qi.x + bm.x + c.x > 0.f) s0 += d.x;
+        if (keep && pj.y + qi.y + bm.y + c.y > 0.f) s1 += d.y;
     }
-    dC[(size_t)e * 64 + f] = s0;
-    dC[(size_t)e * 64 + f + 1] = s1;
+    *reinterpret_cast<float2*>(dC + (size_t)e * 64 + f) = make_float2(s0, s1);
 }
 
 // C[e] = Estatic[e] (4 features) . We[4 x 64] (fp32, edge-wise).
@@ -530,17 +603,19 @@ __global__ void edgeProjectKernel(int nEdges, const float* Es, const float* We, 
     C[i] = s;
 }
 
-// dWe[4 x 64] = Es^T dC, dbmsg[64] = column sums of dC.  One CTA per 8 columns: thread t sums the edges t, t + 256,
-// t + 512, ... in that order (two 16-byte loads of dC and one of Es per edge), then a fixed-shape tree adds the 256
-// partial sums, so the result does not depend on timing.
-constexpr int EPB_THREADS = 256;
-__global__ void __launch_bounds__(EPB_THREADS) edgeProjectBackwardKernel(int nEdges, const float* __restrict__ Es,
-                                                                          const float* __restrict__ dC, float* dWe,
-                                                                          float* dbmsg) {
+// dWe[4 x 64] = Es^T dC, dbmsg[64] = column sums of dC.  A cluster of 8 CTAs per 8 columns: thread t of CTA r sums the edges
+// r * 256 + t, then every 2,048th after it, in that order (two 16-byte loads of dC and one of Es per edge), a fixed-shape
+// tree adds a CTA's 256 partial sums and the cluster's first CTA the 8 CTAs' in rank order through distributed shared
+// memory, so the result does not depend on timing.  (One CTA per 8 columns left 140 SMs idle and walked 125 dependent
+// iterations on the 9,241-bus grid's 32,000 edges.)
+constexpr int EPB_THREADS = 256, EPB_CLUSTER = 8;
+__global__ void __cluster_dims__(EPB_CLUSTER, 1, 1) __launch_bounds__(EPB_THREADS)
+    edgeProjectBackwardKernel(int nEdges, const float* __restrict__ Es, const float* __restrict__ dC, float* dWe, float* dbmsg) {
     __shared__ float part[40][EPB_THREADS];   // (k, column) x thread
-    const int t = threadIdx.x, f0 = blockIdx.x * 8;
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int t = threadIdx.x, rank = (int)cluster.block_rank(), f0 = blockIdx.x / EPB_CLUSTER * 8;
     float acc[5][8] = {};
-    for (int e = t; e < nEdges; e += EPB_THREADS) {
+    for (int e = rank * EPB_THREADS + t; e < nEdges; e += EPB_CLUSTER * EPB_THREADS) {
         const float4 es = *reinterpret_cast<const float4*>(Es + (size_t)e * 4);
         const float4 c0 = *reinterpret_cast<const float4*>(dC + (size_t)e * 64 + f0);
         const float4 c1 = *reinterpret_cast<const float4*>(dC + (size_t)e * 64 + f0 + 4);
@@ -563,11 +638,15 @@ __global__ void __launch_bounds__(EPB_THREADS) edgeProjectBackwardKernel(int nEd
             for (int q = 0; q < 40; q++) part[q][t] += part[q][t + stride];
         __syncthreads();
     }
-    if (t < 40) {
+    cluster.sync();
+    if (rank == 0 && t < 40) {
+        float s = 0.f;
+        for (int r = 0; r < EPB_CLUSTER; r++) s += *cluster.map_shared_rank(&part[t][0], r);
         const int k = t / 8, j = t % 8;
-        if (k < 4) dWe[k * 64 + f0 + j] = part[t][0];
-        else dbmsg[f0 + j] = part[t][0];
+        if (k < 4) dWe[k * 64 + f0 + j] = s;
+        else dbmsg[f0 + j] = s;
     }
+    cluster.sync();   // the other CTAs' shared memory is read until here
 }
 
 // dz = dOut * [z > 0] (relu) or dOut, stored bf16 [M x N] from fp32 [M x ldd]; optionally adds dOut to accum.
@@ -765,6 +844,20 @@ extern "C" int olfgpu_gnn_gemm(int M, int K1, int K2, int N, const void* A1, con
     });
 }
 
+extern "C" int olfgpu_gnn_gemm_grad(int M, int K, int N, const void* A, const void* W, float* accum, float* second,
+                                    const void* z, void* dz, void* stream) {
+    return gnnGuard([&] {
+        if (!A || !W || !accum || (N > 64 && !second) || (dz && !z)) throw std::runtime_error("null operand");
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        auto a = static_cast<const __nv_bfloat16*>(A);
+        auto w = static_cast<const __nv_bfloat16*>(W);
+        const GradOut go{accum, second, static_cast<const __nv_bfloat16*>(z), static_cast<__nv_bfloat16*>(dz)};
+        if (K == 64 && N == 128) launchGemmTc<64, 0, 128, true>(M, a, nullptr, w, nullptr, 0, nullptr, nullptr, nullptr, N, nullptr, st, go);
+        else if (K == 128 && N == 64) launchGemmTc<128, 0, 64, true>(M, a, nullptr, w, nullptr, 0, nullptr, nullptr, nullptr, N, nullptr, st, go);
+        else throw std::runtime_error("unsupported gradient GEMM shape");
+    });
+}
+
 extern "C" int olfgpu_gnn_gemm_dw(int M, int K1, int K2, int N, const void* A1, const void* A2, const void* dZ,
                                   float* dW, float* db, float* partial, int maxChunks, void* stream) {
     return gnnGuard([&] {
@@ -801,19 +894,48 @@ extern "C" int olfgpu_gnn_message_forward(int B, int nb, const int* inPtr, const
     });
 }
 
+namespace {
+void messageBackward(int B, int nb, int nEdges, const int* inPtr, const int* inEdge, const int* outPtr, const int* outEdge,
+                     const int* edgeSrc, const int* edgeDst, const int* edgeBranch, const int* outage, const void* PQ,
+                     const float* C, const float* bmsg, const float* dAgg, float* dPQ, void* dPQb, float* dC, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const long long warps = (long long)B * nb;
+    auto pq = static_cast<const __nv_bfloat16*>(PQ);
+    const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
+    if (dPQ) {
+        messageBackwardNodesKernel<float><<<grid, 256, 0, st>>>(B, nb, inPtr, inEdge, outPtr, outEdge, edgeSrc, edgeDst,
+                                                                edgeBranch, outage, pq, C, bmsg, dAgg, dPQ);
+    } else {
+        messageBackwardNodesKernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
+            B, nb, inPtr, inEdge, outPtr, outEdge, edgeSrc, edgeDst, edgeBranch, outage, pq, C, bmsg, dAgg,
+            static_cast<__nv_bfloat16*>(dPQb));
+    }
+    messageBackwardEdgesKernel<<<(unsigned)(((long long)nEdges * 32 + 255) / 256), 256, 0, st>>>(
+        B, nb, nEdges, edgeSrc, edgeDst, edgeBranch, outage, pq, C, bmsg, dAgg, dC);
+}
+}  // namespace
+
 extern "C" int olfgpu_gnn_message_backward(int B, int nb, int nEdges, const int* inPtr, const int* inEdge,
                                            const int* outPtr, const int* outEdge, const int* edgeSrc,
                                            const int* edgeDst, const int* edgeBranch, const int* outage,
                                            const void* PQ, const float* C, const float* bmsg, const float* dAgg,
                                            float* dPQ, float* dC, void* stream) {
     return gnnGuard([&] {
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        const long long warps = (long long)B * nb;
-        auto pq = static_cast<const __nv_bfloat16*>(PQ);
-        messageBackwardNodesKernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(
-            B, nb, inPtr, inEdge, outPtr, outEdge, edgeSrc, edgeDst, edgeBranch, outage, pq, C, bmsg, dAgg, dPQ);
-        messageBackwardEdgesKernel<<<(unsigned)(((long long)nEdges * 32 + 255) / 256), 256, 0, st>>>(
-            B, nb, nEdges, edgeSrc, edgeDst, edgeBranch, outage, pq, C, bmsg, dAgg, dC);
+        if (!dPQ) throw std::runtime_error("null output");
+        messageBackward(B, nb, nEdges, inPtr, inEdge, outPtr, outEdge, edgeSrc, edgeDst, edgeBranch, outage, PQ, C, bmsg,
+                        dAgg, dPQ, nullptr, dC, stream);
+    });
+}
+
+extern "C" int olfgpu_gnn_message_backward_bf16(int B, int nb, int nEdges, const int* inPtr, const int* inEdge,
+                                                const int* outPtr, const int* outEdge, const int* edgeSrc,
+                                                const int* edgeDst, const int* edgeBranch, const int* outage,
+                                                const void* PQ, const float* C, const float* bmsg, const float* dAgg,
+                                                void* dPQ, float* dC, void* stream) {
+    return gnnGuard([&] {
+        if (!dPQ) throw std::runtime_error("null output");
+        messageBackward(B, nb, nEdges, inPtr, inEdge, outPtr, outEdge, edgeSrc, edgeDst, edgeBranch, outage, PQ, C, bmsg,
+                        dAgg, nullptr, dPQ, dC, stream);
     });
 }
 
@@ -828,7 +950,7 @@ extern "C" int olfgpu_gnn_edge_project_backward(int nEdges, const float* Es, con
     return gnnGuard([&] {
         if ((reinterpret_cast<uintptr_t>(Es) | reinterpret_cast<uintptr_t>(dC)) & 15)
             throw std::runtime_error("edge features and their gradients must be 16-byte aligned");
-        edgeProjectBackwardKernel<<<64 / 8, EPB_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(nEdges, Es, dC, dWe,
+        edgeProjectBackwardKernel<<<64 / 8 * EPB_CLUSTER, EPB_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(nEdges, Es, dC, dWe,
                                                                                                  dbmsg);
     });
 }

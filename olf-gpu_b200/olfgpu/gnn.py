@@ -39,8 +39,10 @@ def _lib():
             "olfgpu_gnn_gemm": [i, i, i, i, vp, vp, vp, vp, i, vp, vp, vp, i, vp, vp],
             "olfgpu_gnn_tc_timeouts": [vp],
             "olfgpu_gnn_gemm_dw": [i, i, i, i, vp, vp, vp, vp, vp, vp, i, vp],
+            "olfgpu_gnn_gemm_grad": [i, i, i, vp, vp, vp, vp, vp, vp, vp],
             "olfgpu_gnn_message_forward": [i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
             "olfgpu_gnn_message_backward": [i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
+            "olfgpu_gnn_message_backward_bf16": [i, i, i, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
             "olfgpu_gnn_edge_project": [i, vp, vp, vp, vp],
             "olfgpu_gnn_edge_project_backward": [i, vp, vp, vp, vp, vp],
             "olfgpu_gnn_relu_grad": [ctypes.c_longlong, i, i, vp, vp, vp, vp, vp],
@@ -307,38 +309,32 @@ class WarmStartNet:
         dh = torch.empty((M, H), dtype=torch.float32, device=self.dev)
         _call("olfgpu_gnn_gemm", M, FEAT_OUT, 0, H, _ptr(dzo), None, _ptr(self.wt["w_out"]), None, 0, None, None,
               _ptr(dh), H, None, st)
-        tmp2 = torch.empty((M, 2 * H), dtype=torch.float32, device=self.dev)
-        tmp = torch.empty((M, H), dtype=torch.float32, device=self.dev)
         dagg = torch.empty((M, H), dtype=torch.float32, device=self.dev)
+        dz = torch.empty((M, H), dtype=bf, device=self.dev)
+        _call("olfgpu_gnn_relu_grad", M * H, H, H, _ptr(dh), _ptr(s["z"][-1] if self.layers else s["h"][0]), _ptr(dz),
+              None, st)
+        dpq = torch.empty((M, 2 * H), dtype=bf, device=self.dev)
         for l in reversed(range(self.layers)):
-            h_l, agg, pq, z, c = s["h"][l], s["agg"][l], s["pq"][l], s["z"][l], s["c"][l]
-            dz = torch.empty((M, H), dtype=bf, device=self.dev)
-            _call("olfgpu_gnn_relu_grad", M * H, H, H, _ptr(dh), _ptr(z), _ptr(dz), None, st)
+            h_l, agg, pq, c = s["h"][l], s["agg"][l], s["pq"][l], s["c"][l]
             self._dw(M, H, H, H, h_l, agg, dz, f"w_upd{l}", f"b_upd{l}")
-            _call("olfgpu_gnn_gemm", M, H, 0, 2 * H, _ptr(dz), None, _ptr(self.wt[f"w_upd{l}"]), None, 0, None, None,
-                  _ptr(tmp2), 2 * H, None, st)
-            # residual: dh stays; the [h | agg] halves of the update's input gradient split off
-            _call("olfgpu_gnn_copy_cols", M, H, _ptr(tmp2), 2 * H, 0, _ptr(dh), H, 0, 1, st)
-            _call("olfgpu_gnn_copy_cols", M, H, _ptr(tmp2), 2 * H, H, _ptr(dagg), H, 0, 0, st)
-            dpq = torch.empty((M, 2 * H), dtype=torch.float32, device=self.dev)
+            # the residual: dh stays and takes the h half of the update's input gradient, dagg is the other half
+            _call("olfgpu_gnn_gemm_grad", M, H, 2 * H, _ptr(dz), _ptr(self.wt[f"w_upd{l}"]), _ptr(dh), _ptr(dagg), None,
+                  None, st)
             dc = torch.empty((g.n_edges, H), dtype=torch.float32, device=self.dev)
-            _call("olfgpu_gnn_message_backward", B, g.nb, g.n_edges, _ptr(g.in_ptr), _ptr(g.in_edge), _ptr(g.out_ptr),
-                  _ptr(g.out_edge), _ptr(g.src), _ptr(g.dst), _ptr(g.branch), _ptr(s["outage"]), _ptr(pq), _ptr(c),
-                  _ptr(self.w[f"b_msg{l}"]), _ptr(dagg), _ptr(dpq), _ptr(dc), st)
+            _call("olfgpu_gnn_message_backward_bf16", B, g.nb, g.n_edges, _ptr(g.in_ptr), _ptr(g.in_edge),
+                  _ptr(g.out_ptr), _ptr(g.out_edge), _ptr(g.src), _ptr(g.dst), _ptr(g.branch), _ptr(s["outage"]),
+                  _ptr(pq), _ptr(c), _ptr(self.w[f"b_msg{l}"]), _ptr(dagg), _ptr(dpq), _ptr(dc), st)
             gwe = torch.empty((4, H), dtype=torch.float32, device=self.dev)
             gbm = torch.empty((1, H), dtype=torch.float32, device=self.dev)
             _call("olfgpu_gnn_edge_project_backward", g.n_edges, _ptr(g.es), _ptr(dc), _ptr(gwe), _ptr(gbm), st)
             self.grad[f"w_e{l}"] = gwe
             self.grad[f"b_msg{l}"] = gbm
-            dpqb = torch.empty((M, 2 * H), dtype=bf, device=self.dev)
-            _call("olfgpu_gnn_relu_grad", M * 2 * H, 2 * H, 2 * H, _ptr(dpq), None, _ptr(dpqb), None, st)
-            self._dw(M, H, 0, 2 * H, h_l, None, dpqb, f"w_pq{l}", None)
-            _call("olfgpu_gnn_gemm", M, 2 * H, 0, H, _ptr(dpqb), None, _ptr(self.wt[f"w_pq{l}"]), None, 0, None, None,
-                  _ptr(tmp), H, None, st)
-            _call("olfgpu_gnn_copy_cols", M, H, _ptr(tmp), H, 0, _ptr(dh), H, 0, 1, st)
-        dz0 = torch.empty((M, H), dtype=bf, device=self.dev)
-        _call("olfgpu_gnn_relu_grad", M * H, H, H, _ptr(dh), _ptr(s["h"][0]), _ptr(dz0), None, st)
-        self._dw(M, FEAT_IN, 0, H, s["x0"], None, dz0, "w_in", "b_in")
+            self._dw(M, H, 0, 2 * H, h_l, None, dpq, f"w_pq{l}", None)
+            # dh is complete for this layer: the ReLU below it (the previous layer's, or the input projection's) is
+            # applied in the same pass
+            _call("olfgpu_gnn_gemm_grad", M, 2 * H, H, _ptr(dpq), _ptr(self.wt[f"w_pq{l}"]), _ptr(dh), None,
+                  _ptr(s["z"][l - 1] if l else s["h"][0]), _ptr(dz), st)
+        self._dw(M, FEAT_IN, 0, H, s["x0"], None, dz, "w_in", "b_in")
         return self.grad
 
     def loss_and_grad(self, x0, outage, target):

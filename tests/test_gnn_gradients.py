@@ -1,0 +1,64 @@
+"""The gradient GEMM with its fused accumulation and ReLU, the BF16 message gradient and the clustered edge-weight gradient
+against float64 references, at the edges of the 128-row tiles."""
+import numpy as np
+import pytest
+
+from conftest import grid
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 127, 128, 129, 128 * 1500 + 3])
+@pytest.mark.parametrize("k,n", [(64, 128), (128, 64)])
+def test_gradient_gemm_matches_float64(engine_lib, k, n, M):
+    """accum += A W[:, :64] in FP32, second = A W[:, 64:], dz = the new accum where z > 0.  FP32 sums of k BF16 products:
+    k * 2^-24 relative to the largest, 1e-5 leaves a margin; dz adds BF16's 2^-9."""
+    import torch
+    from olfgpu import gnn
+    rng = np.random.default_rng(M + k)
+    A = torch.from_numpy(rng.standard_normal((M, k)).astype(np.float32)).cuda().to(torch.bfloat16)
+    W = torch.from_numpy((rng.standard_normal((k, n)) / 8).astype(np.float32)).cuda().to(torch.bfloat16)
+    z = torch.from_numpy(rng.standard_normal((M, 64)).astype(np.float32)).cuda().to(torch.bfloat16)
+    acc0 = torch.from_numpy(rng.standard_normal((M, 64)).astype(np.float32)).cuda()
+    acc, dz = acc0.clone(), torch.empty((M, 64), dtype=torch.bfloat16, device="cuda")
+    second = torch.empty((M, 64), dtype=torch.float32, device="cuda") if n == 128 else None
+    gnn._call("olfgpu_gnn_gemm_grad", M, k, n, gnn._ptr(A), gnn._ptr(W), gnn._ptr(acc), gnn._ptr(second), gnn._ptr(z),
+              gnn._ptr(dz), gnn._stream())
+    y = A.double() @ W.double()
+    ref = acc0.double() + y[:, :64]
+    scale = float(ref.abs().max())
+    assert float((acc.double() - ref).abs().max()) / scale < 1e-5
+    if n == 128:
+        assert float((second.double() - y[:, 64:]).abs().max()) / float(y.abs().max()) < 1e-5
+    want = torch.where(z > 0, acc, torch.zeros_like(acc)).to(torch.bfloat16)
+    assert torch.equal(dz, want)
+    assert gnn.tc_timeouts() == 0
+
+
+@pytest.mark.parametrize("B", [1, 3, 9])
+def test_message_gradients_match(engine_lib, B):
+    """dPQ rounded to BF16 is the FP32 entry's dPQ rounded; the edge-weight gradient is the float64 product."""
+    import torch
+    from olfgpu import gnn
+    g, _ = grid("grid118")
+    gd = gnn.GraphData.from_grid(g)
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    M = B * gd.nb
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    pq, C, bm, dagg = rnd(M, 128).to(torch.bfloat16), rnd(gd.n_edges, 64), rnd(64), rnd(M, 64)
+    outage = torch.arange(B, dtype=torch.int32, device="cuda") * 5
+    d32 = torch.empty((M, 128), device="cuda")
+    d16 = torch.empty((M, 128), dtype=torch.bfloat16, device="cuda")
+    dc32, dc16 = torch.empty((gd.n_edges, 64), device="cuda"), torch.empty((gd.n_edges, 64), device="cuda")
+    for name, out, dc in (("olfgpu_gnn_message_backward", d32, dc32), ("olfgpu_gnn_message_backward_bf16", d16, dc16)):
+        gnn._call(name, B, gd.nb, gd.n_edges, *[gnn._ptr(t) for t in (gd.in_ptr, gd.in_edge, gd.out_ptr, gd.out_edge, gd.src,
+                  gd.dst, gd.branch, outage, pq, C, bm, dagg, out, dc)], gnn._stream())
+    assert torch.equal(d16, d32.to(torch.bfloat16)) and torch.equal(dc16, dc32)
+    we, db = torch.empty((4, 64), device="cuda"), torch.empty((1, 64), device="cuda")
+    gnn._call("olfgpu_gnn_edge_project_backward", gd.n_edges, gnn._ptr(gd.es), gnn._ptr(dc32), gnn._ptr(we), gnn._ptr(db),
+              gnn._stream())
+    ref, refb = gd.es.double().T @ dc32.double(), dc32.double().sum(0)
+    # FP32 sums over n_edges terms: n_edges * 2^-24 of the terms' magnitudes
+    bound = gd.n_edges * 2.0 ** -24
+    assert float((we - ref).abs().max()) <= bound * float((gd.es.abs().T @ dc32.abs()).max())
+    assert float((db[0] - refb).abs().max()) <= bound * float(dc32.abs().sum(0).max())
