@@ -862,15 +862,18 @@ bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cu
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    // (below four chunks the threads cost what they save)
-    if (pageable && bytes >= 4 * CHUNK && !ring) {
+    // (below two chunks the threads cost what they save; pinning the ring costs 3 ms, which a first copy under 16 MiB would
+    // not earn back)
+    const bool again = seen || bytes >= 32 * CHUNK;
+    seen = true;
+    if (pageable && bytes >= 2 * CHUNK && !ring && again) {
         if (cudaMallocHost(&ring, SLOTS * CHUNK) != cudaSuccess) {
             cudaGetLastError();
             ring = nullptr;
         }
         for (cudaEvent_t& e : ready) OLF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
-    if (!pageable || bytes < 4 * CHUNK || !ring) {
+    if (!pageable || bytes < 2 * CHUNK || !ring) {
         OLF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         return true;
     }

@@ -27,6 +27,8 @@
 #include "kernels.cuh"
 
 #include <algorithm>
+#include <map>
+#include <utility>
 
 #include "multifrontal.hpp"
 
@@ -894,11 +896,18 @@ MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int n
             while (G > 1 && teamBytes(n, G, elem, factor) > MF_SHARE_BYTES) G /= 2;
             return G;
         };
+        std::map<std::pair<int, int>, std::pair<int, int>> shapes;      // (p, q): a node of that shape, how many
+        for (int x = firstTeam; x < ptr[l + 1]; x++) {
+            const MfNode& n = plan.node[order[x]];
+            auto& e = shapes[{n.p, n.q}];
+            e.first = order[x];
+            e.second++;
+        }
         auto ctas = [&] {
             long c = 0;
-            for (int x = firstTeam; x < ptr[l + 1]; x++) {
-                const int G = pairs(plan.node[order[x]], cap);
-                c += (nP + G - 1) / G;
+            for (const auto& e : shapes) {
+                const int G = pairs(plan.node[e.second.first], cap);
+                c += (long)e.second.second * ((nP + G - 1) / G);
             }
             return c;
         };

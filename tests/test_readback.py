@@ -1,5 +1,5 @@
 """Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's threshold
-and its chunk size (2 MiB, from 8 MiB on)."""
+(1 MiB), its chunks (512 KiB) and more chunks than its slots."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,7 @@ from conftest import grid
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("count", [1, 261, 262, 263, 328, 1049])
+@pytest.mark.parametrize("count", [1, 32, 33, 49, 131, 132, 1049])
 def test_pageable_results_equal_pinned_ones(engine_lib, count):
     import torch
     from olfgpu import native, synthetic
@@ -19,8 +19,9 @@ def test_pageable_results_equal_pinned_ones(engine_lib, count):
     dis = p.outage_masks(synthetic.draw_outages(g, count, seed=3))
     pinned = torch.empty((count, p.n + 3), dtype=torch.float64).pin_memory().numpy()
     ctx.solve(p.x_base, p.target, p.base_row_mode, dis, out=pinned)
-    fresh = ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
-    assert np.array_equal(fresh, pinned, equal_nan=True)
+    for _ in range(2):          # a small result's first copy is direct
+        fresh = ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
+        assert np.array_equal(fresh, pinned, equal_nan=True)
 
 
 def test_security_analysis_writes_chunks_in_place(engine_lib):
