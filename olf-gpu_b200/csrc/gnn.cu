@@ -347,9 +347,17 @@ void launchGemmTc(int M, const __nv_bfloat16* a1, const __nv_bfloat16* a2, const
 }
 
 // Partial weight gradients: chunk c of the rows contributes P_c[K x N] = [A1|A2]_c^T dZ_c and colsum(dZ_c); one CTA
-// per chunk.  32-row slices stream through two shared-memory buffers with cp.async (16-byte copies, rows past the
-// chunk zero-filled), the next slice in flight while the tensor-core tiles (m over K, n over N, k over rows) consume
-// the current one.
+// per chunk.  32-row slices stream through three shared-memory buffers with cp.async (16-byte copies, rows past the
+// chunk zero-filled), two slices in flight while the tensor-core tiles (m over K, n over N, k over rows) consume
+// the current one.  Both operands are transposed on their way to the registers (ldmatrix.trans): an A tile serves a row
+// of n tiles and one load brings the B fragments of two, 6 loads for 16 MMAs instead of 12 two-byte loads for each.
+__device__ __forceinline__ void ldmatrix4t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
 template <int K1, int K2, int N>
 __global__ void __launch_bounds__(128) gemmDwKernel(int M, int rowsPerChunk, const __nv_bfloat16* __restrict__ A1,
                                                     const __nv_bfloat16* __restrict__ A2,
@@ -358,87 +366,94 @@ __global__ void __launch_bounds__(128) gemmDwKernel(int M, int rowsPerChunk, con
     constexpr int MT = K / 16, NT = N / 8, TILES = MT * NT;
     constexpr int PER_WARP = (TILES + 3) / 4;
     constexpr int SR = 32;                              // rows per slice
-    __shared__ __align__(16) __nv_bfloat16 as[2][SR][K + 8];
-    __shared__ __align__(16) __nv_bfloat16 ds[2][SR][N + 8];
+    constexpr int BUFS = 3;
+    static_assert(TILES % 4 == 0 && PER_WARP % 2 == 0 && (PER_WARP % NT == 0 || NT % PER_WARP == 0), "tiles of a warp: whole rows or a part of one");
+    __shared__ __align__(16) __nv_bfloat16 as[BUFS][SR][K + 8];
+    __shared__ __align__(16) __nv_bfloat16 ds[BUFS][SR][N + 8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int row0 = blockIdx.x * rowsPerChunk;
     const int row1 = min(M, row0 + rowsPerChunk);
     auto stage = [&](int base, int buf) {
-        for (int i = threadIdx.x; i < SR * (K / 8); i += 128) {
-            const int r = i / (K / 8), c = i % (K / 8), row = base + r;
-            const bool valid = row < row1;
-            const size_t rr = valid ? (size_t)row : (size_t)row0;
-            const __nv_bfloat16* src = c * 8 < K1 ? A1 + rr * K1 + c * 8 : A2 + rr * K2 + (c * 8 - K1);
-            cpAsync16(smemU32(&as[buf][r][c * 8]), src, valid);
+        if (base < row1) {
+            for (int i = threadIdx.x; i < SR * (K / 8); i += 128) {
+                const int r = i / (K / 8), c = i % (K / 8), row = base + r;
+                const bool valid = row < row1;
+                const size_t rr = valid ? (size_t)row : (size_t)row0;
+                const __nv_bfloat16* src = c * 8 < K1 ? A1 + rr * K1 + c * 8 : A2 + rr * K2 + (c * 8 - K1);
+                cpAsync16(smemU32(&as[buf][r][c * 8]), src, valid);
+            }
+            for (int i = threadIdx.x; i < SR * (N / 8); i += 128) {
+                const int r = i / (N / 8), c = i % (N / 8), row = base + r;
+                const bool valid = row < row1;
+                cpAsync16(smemU32(&ds[buf][r][c * 8]), dZ + (valid ? (size_t)row : (size_t)row0) * N + c * 8, valid);
+            }
         }
-        for (int i = threadIdx.x; i < SR * (N / 8); i += 128) {
-            const int r = i / (N / 8), c = i % (N / 8), row = base + r;
-            const bool valid = row < row1;
-            cpAsync16(smemU32(&ds[buf][r][c * 8]), dZ + (valid ? (size_t)row : (size_t)row0) * N + c * 8, valid);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");   // (an empty group past the chunk's end)
     };
     float acc[PER_WARP][4];
 #pragma unroll
     for (int i = 0; i < PER_WARP; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     float colsum = 0.f;   // thread tid < N sums column tid of dZ
-    if (row0 < row1) stage(row0, 0);
+    // this lane's row of the four 8x8 matrices of an A tile (k by (lane >> 4), m by (lane >> 3) & 1) and of two B tiles
+    const int ak = (lane >> 4) * 8 + (lane & 7), am = ((lane >> 3) & 1) * 8;
+    const int bk = ((lane >> 3) & 1) * 8 + (lane & 7), bn = (lane >> 4) * 8;
+    stage(row0, 0);
+    stage(row0 + SR, 1);
     int buf = 0;
-    for (int base = row0; base < row1; base += SR, buf ^= 1) {
-        // the other buffer was consumed in the previous slice, before its closing barrier
-        if (base + SR < row1) {
-            stage(base + SR, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
+    for (int base = row0; base < row1; base += SR) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();    // this slice has landed, and every thread is done with the buffer staged next
+        stage(base + 2 * SR, buf >= 1 ? buf - 1 : BUFS - 1);
         if (threadIdx.x < N) {
+#pragma unroll 8
             for (int r = 0; r < SR; r++) colsum += __bfloat162float(ds[buf][r][threadIdx.x]);
         }
 #pragma unroll
         for (int s0 = 0; s0 < SR; s0 += 16) {
-            const __nv_bfloat16(*a16)[K + 8] = &as[buf][s0];
-            const __nv_bfloat16(*d16)[N + 8] = &ds[buf][s0];
+            uint32_t a[4];
 #pragma unroll
-            for (int i = 0; i < PER_WARP; i++) {
+            for (int i = 0; i < PER_WARP; i += 2) {
                 const int tile = warp * PER_WARP + i;
-                if (tile >= TILES) break;
                 const int m0 = (tile / NT) * 16, n0 = (tile % NT) * 8;
-                uint32_t a[4], b[2];
-                // A_mma(m, kk) = a16[kk][m0 + m]; B_mma(kk, n) = d16[kk][n0 + n]
-                a[0] = pack2(a16[2 * t][m0 + g], a16[2 * t + 1][m0 + g]);
-                a[1] = pack2(a16[2 * t][m0 + g + 8], a16[2 * t + 1][m0 + g + 8]);
-                a[2] = pack2(a16[2 * t + 8][m0 + g], a16[2 * t + 9][m0 + g]);
-                a[3] = pack2(a16[2 * t + 8][m0 + g + 8], a16[2 * t + 9][m0 + g + 8]);
-                b[0] = pack2(d16[2 * t][n0 + g], d16[2 * t + 1][n0 + g]);
-                b[1] = pack2(d16[2 * t + 8][n0 + g], d16[2 * t + 9][n0 + g]);
-                mma16816(acc[i], a, b);
+                if (i % NT == 0) ldmatrix4t(a, smemU32(&as[buf][s0 + ak][m0 + am]));
+                uint32_t bb[4];
+                ldmatrix4t(bb, smemU32(&ds[buf][s0 + bk][n0 + bn]));
+                const uint32_t b0[2] = {bb[0], bb[1]}, b1[2] = {bb[2], bb[3]};
+                mma16816(acc[i], a, b0);
+                mma16816(acc[i + 1], a, b1);
             }
         }
-        __syncthreads();
+        buf = buf + 1 == BUFS ? 0 : buf + 1;
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     float* out = partial + (size_t)blockIdx.x * (K * N + N);
 #pragma unroll
     for (int i = 0; i < PER_WARP; i++) {
         const int tile = warp * PER_WARP + i;
-        if (tile >= TILES) break;
         const int m0 = (tile / NT) * 16, n0 = (tile % NT) * 8;
-        out[(m0 + g) * N + n0 + 2 * t] = acc[i][0];
-        out[(m0 + g) * N + n0 + 2 * t + 1] = acc[i][1];
-        out[(m0 + g + 8) * N + n0 + 2 * t] = acc[i][2];
-        out[(m0 + g + 8) * N + n0 + 2 * t + 1] = acc[i][3];
+        *reinterpret_cast<float2*>(out + (m0 + g) * N + n0 + 2 * t) = make_float2(acc[i][0], acc[i][1]);
+        *reinterpret_cast<float2*>(out + (m0 + g + 8) * N + n0 + 2 * t) = make_float2(acc[i][2], acc[i][3]);
     }
     if (threadIdx.x < N) out[K * N + threadIdx.x] = colsum;
 }
 
-// dW[K x N], db[N] = sums of the chunk partials in chunk order.
-__global__ void reducePartialsKernel(int chunks, int KN, int N, const float* partial, float* dW, float* db) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= KN + N) return;
+// dW[K x N], db[N] = sums of the chunk partials: eight strands of consecutive chunks an output, added in strand order (a
+// CTA: 32 outputs x 8 strands).
+__global__ void __launch_bounds__(256) reducePartialsKernel(int chunks, int KN, int N, const float* __restrict__ partial,
+                                                            float* dW, float* db) {
+    __shared__ float part[8][32];
+    const int i = blockIdx.x * 32 + threadIdx.x, k = threadIdx.y;
     float s = 0.f;
-    for (int c = 0; c < chunks; c++) s += partial[(size_t)c * (KN + N) + i];
+    if (i < KN + N) {
+        const int per = (chunks + 7) / 8, c1 = min(chunks, (k + 1) * per);
+#pragma unroll 8
+        for (int c = k * per; c < c1; c++) s += partial[(size_t)c * (KN + N) + i];
+    }
+    part[k][threadIdx.x] = s;
+    __syncthreads();
+    if (k != 0 || i >= KN + N) return;
+    for (int x = 1; x < 8; x++) s += part[x][threadIdx.x];
     if (i < KN) dW[i] = s;
     else if (db) db[i - KN] = s;
 }
@@ -879,7 +894,7 @@ extern "C" int olfgpu_gnn_gemm_dw(int M, int K1, int K2, int N, const void* A1, 
         else throw std::runtime_error("unsupported weight-gradient shape");
 #undef OLF_DW
         const int KN = (K1 + K2) * N;
-        reducePartialsKernel<<<(KN + N + 255) / 256, 256, 0, st>>>(chunks, KN, N, partial, dW, db);
+        reducePartialsKernel<<<(KN + N + 31) / 32, dim3(32, 8), 0, st>>>(chunks, KN, N, partial, dW, db);
     });
 }
 
