@@ -54,6 +54,18 @@ def test_message_gradients_match(engine_lib, B):
         gnn._call(name, B, gd.nb, gd.n_edges, *[gnn._ptr(t) for t in (gd.in_ptr, gd.in_edge, gd.out_ptr, gd.out_edge, gd.src,
                   gd.dst, gd.branch, outage, pq, C, bm, dagg, out, dc)], gnn._stream())
     assert torch.equal(d16, d32.to(torch.bfloat16)) and torch.equal(dc16, dc32)
+    # arrays off the vector accesses' alignment (one element in): the same values
+    off = lambda x: torch.cat([x.reshape(-1)[:1], x.reshape(-1)])[1:]  # noqa: E731
+    agg, agg1 = torch.empty((M, 64), dtype=torch.bfloat16, device="cuda"), torch.empty(M * 64 + 1, dtype=torch.bfloat16, device="cuda")[1:]
+    pq1, c1, bm1, da1 = off(pq), off(C), off(bm), off(dagg)
+    d1, dc1 = torch.empty(M * 128 + 1, device="cuda")[1:], torch.empty(gd.n_edges * 64 + 1, device="cuda")[1:]
+    gnn._call("olfgpu_gnn_message_backward", B, gd.nb, gd.n_edges, *[gnn._ptr(t) for t in (gd.in_ptr, gd.in_edge, gd.out_ptr,
+              gd.out_edge, gd.src, gd.dst, gd.branch, outage, pq1, c1, bm1, da1, d1, dc1)], gnn._stream())
+    assert torch.equal(d1.reshape(M, 128), d32) and torch.equal(dc1.reshape(-1, 64), dc32)
+    for p_, c_, b_, a_ in ((pq, C, bm, agg), (pq1, c1, bm1, agg1)):
+        gnn._call("olfgpu_gnn_message_forward", B, gd.nb, *[gnn._ptr(t) for t in (gd.in_ptr, gd.in_edge, gd.src, gd.branch,
+                  outage, p_, c_, b_, a_)], gnn._stream())
+    assert torch.equal(agg1.reshape(M, 64), agg)
     we, db = torch.empty((4, 64), device="cuda"), torch.empty((1, 64), device="cuda")
     gnn._call("olfgpu_gnn_edge_project_backward", gd.n_edges, gnn._ptr(gd.es), gnn._ptr(dc32), gnn._ptr(we), gnn._ptr(db),
               gnn._stream())
