@@ -8,8 +8,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
-#include <system_error>
-#include <thread>
 
 namespace olfb200 {
 
@@ -850,63 +848,6 @@ std::shared_ptr<DeviceNet> NetStructure::find(int device) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Results to host memory
-// ---------------------------------------------------------------------------------------------------------------
-HostReadback::~HostReadback() {
-    for (cudaEvent_t e : ready)
-        if (e) cudaEventDestroy(e);
-    if (ring) cudaFreeHost(ring);
-}
-
-bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    cudaPointerAttributes at{};
-    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
-    // (below two chunks the threads cost what they save; pinning the ring costs 3 ms, which a first copy under 16 MiB would
-    // not earn back)
-    const bool again = seen || bytes >= 32 * CHUNK;
-    seen = true;
-    if (pageable && bytes >= 2 * CHUNK && !ring && again) {
-        if (cudaMallocHost(&ring, SLOTS * CHUNK) != cudaSuccess) {
-            cudaGetLastError();
-            ring = nullptr;
-        }
-        for (cudaEvent_t& e : ready) OLF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    if (!pageable || bytes < 2 * CHUNK || !ring) {
-        OLF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
-        return true;
-    }
-    const size_t chunks = (bytes + CHUNK - 1) / CHUNK;
-    cudaError_t err[SLOTS] = {};
-    auto work = [&](int slot, int slots) {
-        err[slot] = cudaSetDevice(device);
-        for (size_t c = slot; c < chunks && err[slot] == cudaSuccess; c += slots) {
-            const size_t at0 = c * CHUNK, len = std::min(CHUNK, bytes - at0);
-            unsigned char* pin = ring + static_cast<size_t>(slot) * CHUNK;
-            cudaError_t e = cudaMemcpyAsync(pin, static_cast<const unsigned char*>(src) + at0, len, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaEventRecord(ready[slot], st);
-            if (e == cudaSuccess) e = cudaEventSynchronize(ready[slot]);
-            if (e == cudaSuccess) std::memcpy(static_cast<unsigned char*>(dst) + at0, pin, len);
-            err[slot] = e;
-        }
-    };
-    const int slots = static_cast<int>(std::min<size_t>(chunks, std::min(SLOTS, std::max(1, static_cast<int>(std::thread::hardware_concurrency()) / 2))));
-    std::vector<std::thread> threads;
-    int mine = 0;     // slots whose thread could not be started run here
-    try {
-        for (int k = 1; k < slots; k++) threads.emplace_back(work, k, slots);
-    } catch (const std::system_error&) {
-        mine = static_cast<int>(threads.size()) + 1;
-    }
-    work(0, slots);
-    for (int k = mine; mine > 0 && k < slots; k++) work(k, slots);
-    for (std::thread& t : threads) t.join();
-    for (int k = 0; k < slots; k++) OLF_CUDA(err[k]);
-    return false;
-}
-
-// ---------------------------------------------------------------------------------------------------------------
 // Batch context
 // ---------------------------------------------------------------------------------------------------------------
 BatchContext::~BatchContext() {
@@ -1292,8 +1233,9 @@ void prepareMultifrontal(BatchContext& ctx, int share) {
         if (!schedules->fits()) return;
         // one buffer for both precisions: a context's FP32 and FP64 factorizations never overlap
         const size_t bytes = static_cast<size_t>(std::max(d.mf.updBlocks, 1)) * 4 * ctx.S * 8;
+        const ErrorMark mark;      // (the installs' launches before it are checked at the end of the solve)
         if (cudaMalloc(&ctx.mfUpd.p, bytes) != cudaSuccess) {
-            cudaGetLastError();
+            mark.drop();
             ctx.mfUpd.p = nullptr;
             return;
         }

@@ -10,22 +10,15 @@
 #include <string>
 #include <vector>
 
+#include "cuda_check.hpp"
 #include "kernels.cuh"
 #include "coop.cuh"
 #include "persistent.cuh"
 #include "multifrontal.hpp"
+#include "readback.hpp"
 #include "structure.hpp"
 
 namespace olfb200 {
-
-#define OLF_CUDA(call)                                                                                              \
-    do {                                                                                                            \
-        cudaError_t err_ = (call);                                                                                  \
-        if (err_ != cudaSuccess) {                                                                                  \
-            throw std::runtime_error(std::string("CUDA error ") + cudaGetErrorString(err_) + " at " __FILE__ ":" + \
-                                     std::to_string(__LINE__));                                                     \
-        }                                                                                                           \
-    } while (0)
 
 // A device allocation owned by its holder (freed on destruction; zero-filled on allocation).
 struct DeviceBuffer {
@@ -55,26 +48,6 @@ struct DeviceBuffer {
     T* as() const {
         return static_cast<T*>(p);
     }
-};
-
-// Brings large results to pageable host memory through a small pinned ring, several threads copying out of it (and taking
-// the page faults of a fresh array) while the next chunks cross the bus.  Pinned or small destinations are copied directly.
-// 74 MB of results to a fresh array: 5 ms, against 26 ms for one pageable copy; 4.8 MB: the pageable copy takes 3 ms.
-class HostReadback {
-public:
-    HostReadback() = default;
-    HostReadback(const HostReadback&) = delete;
-    HostReadback& operator=(const HostReadback&) = delete;
-    ~HostReadback();
-    // Stream-ordered after what st holds; true: enqueued on st (the caller synchronises), false: the copy is complete.
-    bool copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st);
-
-private:
-    static constexpr size_t CHUNK = size_t(512) << 10;   // (a 4 MiB ring: pinning 16 MiB cost a new context 5 ms)
-    static constexpr int SLOTS = 8;
-    unsigned char* ring = nullptr;      // pinned, SLOTS chunks, made on the first large or the second smaller copy
-    bool seen = false;
-    cudaEvent_t ready[SLOTS] = {};
 };
 
 // The structure's read-only device data (shared by every context built on it, on one device).

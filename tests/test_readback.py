@@ -1,13 +1,37 @@
 """Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's threshold
-(1 MiB), its chunks (512 KiB) and more chunks than its slots."""
+(1 MiB), its chunks (512 KiB) and more chunks than its slots (GPU); the ring over a stand-in for the CUDA runtime (CPU)."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 
-from conftest import grid
+from conftest import ROOT, grid
 
-pytestmark = pytest.mark.gpu
+CUDA_INCLUDE = os.path.join(os.path.dirname(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"))), "include")
 
 
+@pytest.fixture(scope="module")
+def host_program(tmp_path_factory):
+    if shutil.which("g++") is None or not os.path.exists(os.path.join(CUDA_INCLUDE, "cuda_runtime_api.h")):
+        pytest.skip("no C++ compiler or CUDA headers")
+    exe = str(tmp_path_factory.mktemp("readback") / "readback_host")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-I", CUDA_INCLUDE,
+                           os.path.join(ROOT, "tests", "c", "readback_host.cpp"),
+                           os.path.join(ROOT, "olf-gpu_b200", "csrc", "readback.cpp"), "-pthread", "-ldl", "-o", exe])
+    return exe
+
+
+@pytest.mark.parametrize("case", ["pending", "own", "sizes"])
+def test_ring_over_a_stand_in_runtime(host_program, case):
+    """A launch error from before the copy is still there after it, the copy's own failed calls leave none, and the bytes are
+    the source's."""
+    out = subprocess.run([host_program, case], capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout + out.stderr
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("count", [1, 32, 33, 49, 131, 132, 1049])
 def test_pageable_results_equal_pinned_ones(engine_lib, count):
     import torch
@@ -24,6 +48,7 @@ def test_pageable_results_equal_pinned_ones(engine_lib, count):
         assert np.array_equal(fresh, pinned, equal_nan=True)
 
 
+@pytest.mark.gpu
 def test_security_analysis_writes_chunks_in_place(engine_lib):
     """A last chunk shorter than the others is padded and copied; every row equals the single batch's."""
     from olfgpu import synthetic
