@@ -3,7 +3,7 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -11,10 +11,27 @@
 
 namespace olfb200 {
 
-HostReadback::~HostReadback() {
-    for (cudaEvent_t e : ready)
+HostReadback::~HostReadback() { release(); }
+
+void HostReadback::release() {
+    for (cudaEvent_t& e : ready) {
         if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     if (ring) cudaFreeHost(ring);
+    ring = nullptr;
+}
+
+// The ring and its events, all or none of them; after a failure the direct copies stay.
+void HostReadback::makeRing() {
+    bool ok = cudaMallocHost(reinterpret_cast<void**>(&ring), SLOTS * CHUNK) == cudaSuccess;
+    if (!ok) ring = nullptr;
+    for (int k = 0; ok && k < SLOTS; k++) {
+        ok = cudaEventCreateWithFlags(&ready[k], cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) ready[k] = nullptr;
+    }
+    if (!ok) release();
+    failed = !ok;
 }
 
 bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
@@ -27,12 +44,9 @@ bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cu
     // not earn back)
     const bool again = seen || bytes >= 32 * CHUNK;
     seen = true;
-    if (pageable && bytes >= 2 * CHUNK && !ring && again) {
-        if (cudaMallocHost(reinterpret_cast<void**>(&ring), SLOTS * CHUNK) != cudaSuccess) {
-            mark.drop();
-            ring = nullptr;
-        }
-        for (cudaEvent_t& e : ready) OLF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (pageable && bytes >= 2 * CHUNK && !ring && !failed && again) {
+        makeRing();
+        if (failed) mark.drop();
     }
     if (!pageable || bytes < 2 * CHUNK || !ring) {
         OLF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
@@ -56,8 +70,9 @@ bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cu
     std::vector<std::thread> threads;
     int mine = 0;     // slots whose thread could not be started run here
     try {
+        threads.reserve(slots);
         for (int k = 1; k < slots; k++) threads.emplace_back(work, k, slots);
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {      // std::system_error, std::bad_alloc: the threads that run are joined below
         mine = static_cast<int>(threads.size()) + 1;
     }
     work(0, slots);

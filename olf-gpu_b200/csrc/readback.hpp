@@ -23,8 +23,10 @@ private:
     static constexpr size_t CHUNK = size_t(512) << 10;   // (a 4 MiB ring: pinning 16 MiB cost a new context 5 ms)
     static constexpr int SLOTS = 8;
     unsigned char* ring = nullptr;      // pinned, SLOTS chunks, made on the first large or the second smaller copy
-    bool seen = false;
+    bool seen = false, failed = false;  // failed: the ring could not be made, and is not tried again
     cudaEvent_t ready[SLOTS] = {};
+    void makeRing();
+    void release();
 };
 
 }  // namespace olfb200

@@ -1,10 +1,14 @@
-// HostReadback (csrc/readback.cpp) over a stand-in for the CUDA runtime in host memory: which errors it leaves behind
-// and the bytes it brings.  Usage: readback_host <case>; prints "ok" or what went wrong.
+// HostReadback (csrc/readback.cpp) over a stand-in for the CUDA runtime in host memory: which errors it leaves behind, what it
+// holds after a failure, and the bytes it brings.  Usage: readback_host <case>; prints "ok" or what went wrong.
+#include <dlfcn.h>
+#include <pthread.h>
+
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -12,8 +16,10 @@
 
 namespace {
 thread_local cudaError_t last = cudaSuccess;       // the runtime's last error is per host thread
-std::atomic<int> eventsMade{0}, directCopies{0}, ringCopies{0};
+std::atomic<int> pinned{0}, pinCalls{0}, eventsMade{0}, eventsGone{0}, directCopies{0}, ringCopies{0};
 bool failQuery = false, failPin = false;
+int failEventAt = -1, failThreadAt = -1, failNewAt = -1;
+std::atomic<int> threadCalls{0}, newCalls{0};
 std::mutex copies;
 unsigned char* ringLo = nullptr;
 size_t ringBytes = 0;
@@ -37,21 +43,28 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* at, const void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) {
+    pinCalls++;
     if (failPin) return fail(cudaErrorMemoryAllocation);
     *p = std::malloc(n);
     ringLo = static_cast<unsigned char*>(*p);
     ringBytes = n;
+    pinned++;
     return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {
     std::free(p);
+    pinned--;
     return cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+    if (failEventAt >= 0 && eventsMade == failEventAt) return fail(cudaErrorMemoryAllocation);
     *e = reinterpret_cast<cudaEvent_t>(static_cast<size_t>(++eventsMade));
     return cudaSuccess;
 }
-cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) {
+    eventsGone++;
+    return cudaSuccess;
+}
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return e ? cudaSuccess : fail(cudaErrorInvalidResourceHandle); }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t) {
@@ -61,7 +74,21 @@ cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind
     std::memcpy(dst, src, n);
     return cudaSuccess;
 }
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) {
+    if (failThreadAt >= 0 && threadCalls++ >= failThreadAt) return EAGAIN;
+    using Create = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+    return reinterpret_cast<Create>(dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, x);
 }
+}
+
+void* operator new(size_t n) {
+    if (failNewAt >= 0 && newCalls++ == failNewAt) throw std::bad_alloc();
+    void* p = std::malloc(n ? n : 1);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 namespace {
 constexpr size_t MIB = size_t(1) << 20;
@@ -112,6 +139,61 @@ void ownError() {
     }
 }
 
+// A ring that cannot be pinned: copied directly, tried once, and no event held or lost.
+void pinFails() {
+    failPin = true;
+    {
+        olfb200::HostReadback r;
+        for (int k = 0; k < 4; k++) expect(!copyOnce(r, 20 * MIB), "copy threw");
+        expect(directCopies == 4, "not copied directly");
+        expect(pinCalls == 1, "pinned again after a failure");
+    }
+    expect(eventsMade == eventsGone, "events lost");
+}
+
+// An event that cannot be made: the ring and the events made before it are given back, copied directly.
+void eventFails() {
+    failEventAt = 3;
+    {
+        olfb200::HostReadback r;
+        for (int k = 0; k < 3; k++) expect(!copyOnce(r, 20 * MIB), "copy threw");
+        expect(directCopies == 3, "not copied directly");
+    }
+    expect(pinned == 0, "ring lost");
+    expect(eventsMade == eventsGone, "events lost");
+    expect(last == cudaSuccess, "the copy left an error behind");
+}
+
+// Threads that cannot be started (by the system, or for want of memory): their chunks are copied by the others.
+void threadsFail() {
+    for (int at = 0; at < 8; at++) {
+        olfb200::HostReadback r;
+        failThreadAt = -1;
+        expect(!copyOnce(r, 20 * MIB), "copy threw");
+        threadCalls = 0;
+        failThreadAt = at;
+        expect(!copyOnce(r, 20 * MIB + 5), "copy threw");
+    }
+}
+void memoryFails() {
+    for (int at = 0; at < 12; at++) {
+        olfb200::HostReadback r;
+        std::vector<unsigned char> src(20 * MIB, 7), dst(20 * MIB, 0);
+        pinnedDst = nullptr;
+        r.copy(0, dst.data(), src.data(), src.size(), nullptr);
+        std::memset(dst.data(), 0, dst.size());
+        newCalls = 0;
+        failNewAt = at;
+        try {
+            r.copy(0, dst.data(), src.data(), src.size(), nullptr);
+            failNewAt = -1;
+            expect(src == dst, "bytes differ");
+        } catch (const std::exception&) {
+            failNewAt = -1;      // before any thread ran: an error is as good
+        }
+    }
+}
+
 // Sizes around the threshold, the chunks and the slots.
 void sizes() {
     olfb200::HostReadback r;
@@ -125,6 +207,10 @@ int main(int argc, char** argv) {
     const std::string c = argc > 1 ? argv[1] : "";
     if (c == "pending") pendingError();
     else if (c == "own") ownError();
+    else if (c == "pin") pinFails();
+    else if (c == "event") eventFails();
+    else if (c == "threads") threadsFail();
+    else if (c == "memory") memoryFails();
     else if (c == "sizes") sizes();
     else wrong = "unknown case";
     std::puts(wrong ? wrong : "ok");

@@ -23,10 +23,11 @@ def host_program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["pending", "own", "sizes"])
+@pytest.mark.parametrize("case", ["pending", "own", "sizes", "pin", "event", "threads", "memory"])
 def test_ring_over_a_stand_in_runtime(host_program, case):
     """A launch error from before the copy is still there after it, the copy's own failed calls leave none, and the bytes are
-    the source's."""
+    the source's.  A ring, an event, a thread or memory that cannot be had: nothing is lost, and the copy is made all the
+    same."""
     out = subprocess.run([host_program, case], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
 
