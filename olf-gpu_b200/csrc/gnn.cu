@@ -365,6 +365,16 @@ __device__ __forceinline__ void ldmatrix4t(uint32_t (&r)[4], uint32_t addr) {
                  : "memory");
 }
 
+// Two neighbouring elements: one 8-byte store, or two where the caller's array is not aligned to it.
+__device__ __forceinline__ void storePair(float* p, bool pairs, float a, float b) {
+    if (pairs) {
+        *reinterpret_cast<float2*>(p) = make_float2(a, b);
+    } else {
+        p[0] = a;
+        p[1] = b;
+    }
+}
+
 template <int K1, int K2, int N>
 __global__ void __launch_bounds__(128) gemmDwKernel(int M, int rowsPerChunk, const __nv_bfloat16* __restrict__ A1,
                                                     const __nv_bfloat16* __restrict__ A2,
@@ -435,12 +445,13 @@ __global__ void __launch_bounds__(128) gemmDwKernel(int M, int rowsPerChunk, con
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     float* out = partial + (size_t)blockIdx.x * (K * N + N);
+    const bool pairs = (reinterpret_cast<uintptr_t>(partial) & 7) == 0;      // (every chunk starts at an even element)
 #pragma unroll
     for (int i = 0; i < PER_WARP; i++) {
         const int tile = warp * PER_WARP + i;
         const int m0 = (tile / NT) * 16, n0 = (tile % NT) * 8;
-        *reinterpret_cast<float2*>(out + (m0 + g) * N + n0 + 2 * t) = make_float2(acc[i][0], acc[i][1]);
-        *reinterpret_cast<float2*>(out + (m0 + g + 8) * N + n0 + 2 * t) = make_float2(acc[i][2], acc[i][3]);
+        storePair(out + (m0 + g) * N + n0 + 2 * t, pairs, acc[i][0], acc[i][1]);
+        storePair(out + (m0 + g + 8) * N + n0 + 2 * t, pairs, acc[i][2], acc[i][3]);
     }
     if (threadIdx.x < N) out[K * N + threadIdx.x] = colsum;
 }

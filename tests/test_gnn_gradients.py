@@ -35,6 +35,30 @@ def test_gradient_gemm_matches_float64(engine_lib, k, n, M):
     assert gnn.tc_timeouts() == 0
 
 
+@pytest.mark.parametrize("M", [1, 33, 128 * 5 + 7])
+@pytest.mark.parametrize("k1,k2,n", [(16, 0, 64), (64, 0, 128), (64, 64, 64), (64, 0, 16)])
+def test_weight_gradient_with_partials_off_the_pair_alignment(engine_lib, k1, k2, n, M):
+    """A scratch array that starts at an odd element gives the bits of an aligned one.  Against float64: FP32 sums of M products
+    of BF16 values, M * 2^-24 of the products' magnitudes."""
+    import torch
+    from olfgpu import gnn
+    rng = np.random.default_rng(M + k1 + n)
+    draw = lambda *s: torch.from_numpy(rng.standard_normal(s).astype(np.float32)).cuda().to(torch.bfloat16)  # noqa: E731
+    a1, a2, dz = draw(M, k1), draw(M, k2) if k2 else None, draw(M, n)
+    chunks, k = 3, k1 + k2
+    got = []
+    for first in (0, 1):
+        partial = torch.full((chunks * (k * n + n) + 1,), float("nan"), device="cuda")[first:]
+        dw, db = torch.empty((k, n), device="cuda"), torch.empty(n, device="cuda")
+        gnn._call("olfgpu_gnn_gemm_dw", M, k1, k2, n, gnn._ptr(a1), gnn._ptr(a2), gnn._ptr(dz), gnn._ptr(dw), gnn._ptr(db),
+                  gnn._ptr(partial), chunks, gnn._stream())
+        got.append((dw, db))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    a = torch.cat([a1, a2], 1).double() if k2 else a1.double()
+    assert bool((torch.abs(got[0][0] - a.T @ dz.double()) <= (M + 8) * 2.0 ** -24 * (a.abs().T @ dz.double().abs())).all())
+    assert bool((torch.abs(got[0][1] - dz.double().sum(0)) <= (M + 8) * 2.0 ** -24 * dz.double().abs().sum(0)).all())
+
+
 @pytest.mark.parametrize("B", [1, 3, 9])
 def test_message_gradients_match(engine_lib, B):
     """dPQ rounded to BF16 is the FP32 entry's dPQ rounded; the edge-weight gradient is the float64 product."""
