@@ -1,7 +1,11 @@
 // Results to host memory (see readback.hpp).  Host code over the CUDA runtime only.
 #include "readback.hpp"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <exception>
 #include <thread>
@@ -34,21 +38,31 @@ void HostReadback::makeRing() {
     failed = !ok;
 }
 
+// At least half of the array's pages (fewer than LARGE bytes) have memory behind them already.
+bool HostReadback::inMemory(const void* p, size_t bytes) {
+    const uintptr_t page = static_cast<uintptr_t>(sysconf(_SC_PAGESIZE));
+    const uintptr_t from = reinterpret_cast<uintptr_t>(p) / page * page;
+    const size_t pages = (reinterpret_cast<uintptr_t>(p) + bytes - from + page - 1) / page;
+    unsigned char there[LARGE / 4096 + 2];
+    if (pages > sizeof(there) || mincore(reinterpret_cast<void*>(from), pages * page, there) != 0) return true;
+    size_t n = 0;
+    for (size_t k = 0; k < pages; k++) n += there[k] & 1;
+    return 2 * n >= pages;
+}
+
 bool HostReadback::copy(int device, void* dst, const void* src, size_t bytes, cudaStream_t st) {
     const ErrorMark mark;      // the caller's launches before the copy are checked after it
     cudaPointerAttributes at{};
     const bool known = cudaPointerGetAttributes(&at, dst) == cudaSuccess;
     if (!known) mark.drop();
     const bool pageable = known && at.type == cudaMemoryTypeUnregistered;
-    // (below two chunks the threads cost what they save; pinning the ring costs 3 ms, which a first copy under 16 MiB would
-    // not earn back)
-    const bool again = seen || bytes >= 32 * CHUNK;
-    seen = true;
-    if (pageable && bytes >= 2 * CHUNK && !ring && !failed && again) {
+    const bool worth = pageable && bytes >= 2 * CHUNK && (bytes >= LARGE || !inMemory(dst, bytes));
+    if (worth) due += bytes;
+    if (worth && !ring && !failed && due >= EARNED) {
         makeRing();
         if (failed) mark.drop();
     }
-    if (!pageable || bytes < 2 * CHUNK || !ring) {
+    if (!worth || !ring) {
         OLF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         return true;
     }

@@ -8,8 +8,15 @@
 namespace olfb200 {
 
 // Brings large results to pageable host memory through a small pinned ring, several threads copying out of it (and taking
-// the page faults of a fresh array) while the next chunks cross the bus.  Pinned or small destinations are copied directly.
-// 74 MB of results to a fresh array: 5 ms, against 26 ms for one pageable copy; 4.8 MB: the pageable copy takes 3 ms.
+// the page faults of a fresh array) while the next chunks cross the bus.
+//
+// What it is worth depends on the array.  Fresh pages cost more than the copy, and the threads share them; in an array that
+// is in memory already the threads' start is all that is added, until the copy itself is long enough to share.  Whole solves
+// on 9,241 buses, direct copy / ring, results kept (fresh arrays): 2.4 MiB 3.6 / 3.0 ms, 9.2 MiB 7.4 / 5.9, 18 MiB 10.4 /
+// 6.9; results dropped (the allocator hands out the same pages): 2.4 MiB 2.75 / 3.2 ms, 9.2 MiB 5.9 / 6.8, 18 MiB 7.5 / 7.7,
+// 37 MiB 16.3 / 10.5.  So: fresh arrays from two chunks on (1.1 MiB 2.62 / 2.51 ms), others from EARNED on; pinned memory is
+// copied directly.  Pinning the ring costs 3 to 8 ms once: it is made when the copies it is for have added up to EARNED,
+// about what it saves on them.
 class HostReadback {
 public:
     HostReadback() = default;
@@ -22,9 +29,12 @@ public:
 private:
     static constexpr size_t CHUNK = size_t(512) << 10;   // (a 4 MiB ring: pinning 16 MiB cost a new context 5 ms)
     static constexpr int SLOTS = 8;
-    unsigned char* ring = nullptr;      // pinned, SLOTS chunks, made on the first large or the second smaller copy
-    bool seen = false, failed = false;  // failed: the ring could not be made, and is not tried again
+    static constexpr size_t EARNED = size_t(16) << 20;
+    unsigned char* ring = nullptr;      // pinned, SLOTS chunks
+    size_t due = 0;                     // bytes of the copies that the ring is for, so far
+    bool failed = false;                // the ring could not be made, and is not tried again
     cudaEvent_t ready[SLOTS] = {};
+    static bool inMemory(const void* p, size_t bytes);
     void makeRing();
     void release();
 };

@@ -2,6 +2,7 @@
 // holds after a failure, and the bytes it brings.  Usage: readback_host <case>; prints "ok" or what went wrong.
 #include <dlfcn.h>
 #include <pthread.h>
+#include <sys/mman.h>
 
 #include <atomic>
 #include <cstdio>
@@ -97,18 +98,24 @@ void expect(bool ok, const char* what) {
     if (!ok && !wrong) wrong = what;
 }
 
-// One copy of n bytes; its bytes are compared and whether it threw returned.
-bool copyOnce(olfb200::HostReadback& r, size_t n, bool toPinned = false) {
-    std::vector<unsigned char> src(n), dst(n, 0);
+// One copy of n bytes, to a fresh array or to one whose pages are in memory; its bytes are compared and whether it threw
+// returned.
+enum Kind { FRESH, USED, PINNED };
+bool copyOnce(olfb200::HostReadback& r, size_t n, Kind kind = FRESH) {
+    std::vector<unsigned char> src(n);
     for (size_t i = 0; i < n; i++) src[i] = static_cast<unsigned char>(i * 2654435761u >> 24);
-    pinnedDst = toPinned ? dst.data() : nullptr;
+    unsigned char* dst = static_cast<unsigned char*>(
+        mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+    if (kind != FRESH) std::memset(dst, 0, n);
+    pinnedDst = kind == PINNED ? dst : nullptr;
     bool threw = false;
     try {
-        r.copy(0, dst.data(), src.data(), n, nullptr);
+        r.copy(0, dst, src.data(), n, nullptr);
     } catch (const std::exception&) {
         threw = true;
     }
-    if (!threw) expect(std::memcmp(src.data(), dst.data(), n) == 0, "bytes differ");
+    if (!threw) expect(std::memcmp(src.data(), dst, n) == 0, "bytes differ");
+    munmap(dst, n);
     return threw;
 }
 
@@ -119,9 +126,9 @@ void pendingError() {
         failPin = variant == 2;
         olfb200::HostReadback r;
         for (const size_t n : {MIB / 4, 3 * MIB, 20 * MIB}) {
-            for (const bool toPinned : {false, true}) {
+            for (const Kind kind : {FRESH, USED, PINNED}) {
                 last = cudaErrorInvalidConfiguration;
-                expect(!copyOnce(r, n, toPinned), "copy threw");
+                expect(!copyOnce(r, n, kind), "copy threw");
                 expect(last != cudaSuccess, "a pending launch error was cleared");
             }
         }
@@ -194,12 +201,30 @@ void memoryFails() {
     }
 }
 
-// Sizes around the threshold, the chunks and the slots.
+// Sizes around the thresholds, the chunks and the slots.
 void sizes() {
     olfb200::HostReadback r;
-    for (const size_t n : {size_t(1), MIB / 2, MIB - 1, MIB, MIB + 1, 4 * MIB - 8, 4 * MIB, 4 * MIB + 8, 17 * MIB + 3})
-        for (int k = 0; k < 2; k++) expect(!copyOnce(r, n), "copy threw");
+    for (const size_t n : {size_t(1), MIB / 2, MIB - 1, MIB, MIB + 1, 4 * MIB - 8, 4 * MIB, 4 * MIB + 8, 16 * MIB - 1, 16 * MIB,
+                           17 * MIB + 3})
+        for (const Kind kind : {FRESH, USED, PINNED, FRESH}) expect(!copyOnce(r, n, kind), "copy threw");
     expect(ringCopies > 0, "the ring never ran");
+}
+
+// Which way a copy takes: arrays in memory directly up to 16 MiB, fresh ones through the ring once it has been earned.
+void ways() {
+    olfb200::HostReadback r;
+    auto direct = [&](size_t n, Kind kind) {
+        const int before = directCopies;
+        expect(!copyOnce(r, n, kind), "copy threw");
+        return directCopies == before + 1;
+    };
+    for (int k = 0; k < 20; k++) expect(direct(4 * MIB, USED), "an array in memory went through the ring");
+    expect(pinCalls == 0, "the ring was pinned for arrays in memory");
+    for (int k = 0; k < 3; k++) expect(direct(4 * MIB, FRESH), "the ring was pinned before it was earned");
+    expect(!direct(4 * MIB, FRESH), "a fresh array was copied directly");
+    expect(direct(MIB - 1, FRESH) && direct(4 * MIB, USED) && direct(20 * MIB, PINNED), "a copy went through the ring");
+    expect(!direct(16 * MIB, USED), "a large copy was made directly");
+    expect(pinCalls == 1, "more than one ring");
 }
 }  // namespace
 
@@ -212,6 +237,7 @@ int main(int argc, char** argv) {
     else if (c == "threads") threadsFail();
     else if (c == "memory") memoryFails();
     else if (c == "sizes") sizes();
+    else if (c == "ways") ways();
     else wrong = "unknown case";
     std::puts(wrong ? wrong : "ok");
     return wrong ? 1 : 0;

@@ -1,5 +1,5 @@
-"""Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's threshold
-(1 MiB), its chunks (512 KiB) and more chunks than its slots (GPU); the ring over a stand-in for the CUDA runtime (CPU)."""
+"""Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's thresholds
+(1 and 16 MiB), its chunks (512 KiB) and more chunks than its slots (GPU); the ring over a stand-in for the CUDA runtime (CPU)."""
 import os
 import shutil
 import subprocess
@@ -23,11 +23,12 @@ def host_program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["pending", "own", "sizes", "pin", "event", "threads", "memory"])
+@pytest.mark.parametrize("case", ["pending", "own", "sizes", "pin", "event", "threads", "memory", "ways"])
 def test_ring_over_a_stand_in_runtime(host_program, case):
     """A launch error from before the copy is still there after it, the copy's own failed calls leave none, and the bytes are
     the source's.  A ring, an event, a thread or memory that cannot be had: nothing is lost, and the copy is made all the
-    same."""
+    same.  Arrays in memory are copied directly up to 16 MiB, and the ring is not pinned before the copies it is for add up to
+    that."""
     out = subprocess.run([host_program, case], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
 
@@ -47,6 +48,10 @@ def test_pageable_results_equal_pinned_ones(engine_lib, count):
     for _ in range(2):          # a small result's first copy is direct
         fresh = ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
         assert np.array_equal(fresh, pinned, equal_nan=True)
+    kept = []                   # fresh arrays, through the ring once they add up to 16 MiB
+    for _ in range(0 if count > 500 else 18):
+        kept.append(ctx.solve(p.x_base, p.target, p.base_row_mode, dis))
+        assert np.array_equal(kept[-1], pinned, equal_nan=True)
 
 
 @pytest.mark.gpu
