@@ -204,13 +204,13 @@ void memoryFails() {
 // Sizes around the thresholds, the chunks and the slots.
 void sizes() {
     olfb200::HostReadback r;
-    for (const size_t n : {size_t(1), MIB / 2, MIB - 1, MIB, MIB + 1, 4 * MIB - 8, 4 * MIB, 4 * MIB + 8, 16 * MIB - 1, 16 * MIB,
-                           17 * MIB + 3})
+    for (const size_t n : {size_t(1), MIB / 2, MIB - 1, MIB, MIB + 1, 4 * MIB - 8, 4 * MIB, 4 * MIB + 8, 17 * MIB + 3,
+                           32 * MIB - 1, 32 * MIB, 33 * MIB + 5})
         for (const Kind kind : {FRESH, USED, PINNED, FRESH}) expect(!copyOnce(r, n, kind), "copy threw");
     expect(ringCopies > 0, "the ring never ran");
 }
 
-// Which way a copy takes: arrays in memory directly up to 16 MiB, fresh ones through the ring once it has been earned.
+// Which way a copy takes: arrays in memory directly up to 32 MiB, fresh ones through the ring once it has been earned.
 void ways() {
     olfb200::HostReadback r;
     auto direct = [&](size_t n, Kind kind) {
@@ -223,7 +223,8 @@ void ways() {
     for (int k = 0; k < 3; k++) expect(direct(4 * MIB, FRESH), "the ring was pinned before it was earned");
     expect(!direct(4 * MIB, FRESH), "a fresh array was copied directly");
     expect(direct(MIB - 1, FRESH) && direct(4 * MIB, USED) && direct(20 * MIB, PINNED), "a copy went through the ring");
-    expect(!direct(16 * MIB, USED), "a large copy was made directly");
+    expect(direct(32 * MIB - 1, USED), "an array in memory went through the ring");
+    expect(!direct(32 * MIB, USED), "a large copy was made directly");
     expect(pinCalls == 1, "more than one ring");
 }
 }  // namespace

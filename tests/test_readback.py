@@ -1,5 +1,5 @@
 """Results brought to pageable memory through the pinned ring equal those copied to pinned memory, around the ring's thresholds
-(1 and 16 MiB), its chunks (512 KiB) and more chunks than its slots (GPU); the ring over a stand-in for the CUDA runtime (CPU)."""
+(1, 16 and 32 MiB), its chunks (512 KiB) and more chunks than its slots (GPU); the ring over a stand-in for the CUDA runtime (CPU)."""
 import os
 import shutil
 import subprocess
@@ -27,8 +27,8 @@ def host_program(tmp_path_factory):
 def test_ring_over_a_stand_in_runtime(host_program, case):
     """A launch error from before the copy is still there after it, the copy's own failed calls leave none, and the bytes are
     the source's.  A ring, an event, a thread or memory that cannot be had: nothing is lost, and the copy is made all the
-    same.  Arrays in memory are copied directly up to 16 MiB, and the ring is not pinned before the copies it is for add up to
-    that."""
+    same.  Arrays in memory are copied directly up to 32 MiB, and the ring is not pinned before the copies it is for add up to
+    16 MiB."""
     out = subprocess.run([host_program, case], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
 
