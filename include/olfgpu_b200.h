@@ -111,6 +111,14 @@ int olfgpu_structure_levels(int64_t structure, int* factorLevelPtr, int* forward
 int olfgpu_structure_subtrees(int64_t structure, int64_t* stats6);
 
 /*
+ * The multifrontal plan of the structure's block LU (no counterpart in the reference; schedule 4 of olfgpu_set_schedule
+ * and the FP64 no-allocation solve run it): {nodes, levels of the assembly tree, 2x2 blocks of one lane's update matrices,
+ * rows of the largest front, most rows below a node's pivots} into stats5.  Zeros: no plan, for a grid under 512 buses, a
+ * deferred-L plan, or an elimination order in which some pivot has more than 40 rows below it.
+ */
+int olfgpu_structure_multifrontal(int64_t structure, int64_t* stats5);
+
+/*
  * A host check of the structure's block-LU plan (no counterpart in the reference's API; the reference checks its own
  * LU schedules for races the same way, native/host/lu_transposed_check.cpp:175-216), from the plan's dependency data
  * alone: the symbolic factorization is closed and every block's update list complete and ascending; every LU block is
@@ -260,15 +268,18 @@ int olfgpu_last_fp64_refactors(int64_t context, unsigned char* flagged, int* cou
  * lane holding every LU block those levels produce (lanesPerTile then only sets the solves' narrow-level tiles; plans
  * whose narrow levels do not fit, and deferred-L plans, fall back to schedule 0); schedule 4 is schedule 3 with the
  * solves' narrow levels (the forward tail and the backward head) in shared memory as well, one CTA per lane holding
- * those rows' solution entries (lanesPerTile ignored), or, from 512 buses on, the multifrontal form of the same block LU
- * (one launch per level of its assembly tree; results within rounding); schedule -1 lets the next solve time every candidate on its
- * batch and keep the fastest (the autotuner).  olfgpu_get_schedule reports the schedule in force and, after an
- * autotuned solve, up to maxResults timings {schedule, lanesPerTile, threads, ms} into results (nResults receives
- * their count).
+ * those rows' solution entries (lanesPerTile ignored), or, where the structure has a multifrontal plan
+ * (olfgpu_structure_multifrontal) and the device room for its update matrices at the first solve, the multifrontal form of
+ * the same block LU (one launch per level of its assembly tree; results within rounding); schedule -1 lets the next solve
+ * time every candidate on its batch and keep the fastest (the autotuner).  olfgpu_get_schedule reports the schedule in
+ * force and, after an autotuned solve, up to maxResults timings {schedule, lanesPerTile, threads, ms} into results
+ * (nResults receives their count); olfgpu_multifrontal_in_force whether schedule 4 runs the multifrontal form in this
+ * context (1; 0 otherwise, and before the first solve under it).
  */
 int olfgpu_set_schedule(int64_t context, int schedule, int lanesPerTile, int threads);
 int olfgpu_get_schedule(int64_t context, int* schedule, int* lanesPerTile, int* threads, int maxResults,
                         double* results, int* nResults);
+int olfgpu_multifrontal_in_force(int64_t context, int* inForce);
 
 /*
  * BatchSolveNative.solveBatchContext (batch_solve_jni.cu:84-394; BatchSolveNative.java:106-125).

@@ -257,8 +257,9 @@ extern "C" int olfgpu_structure_check_plan(int64_t structure, int plantedFault, 
         const Structure& s = structureOf(structure)->host;
         const BlockPlan& plan = s.plan;
         *violations = checkBlockPlan(plan, plantedFault, first);
-        if (plantedFault == 0 && !plan.deferredL) {   // the multifrontal form of the same factorization
-            const std::string mf = checkMfPlan(plan, s.nodeCol, buildMfPlan(plan, s.nodeCol));
+        if (plantedFault == 0 && !plan.deferredL) {   // the multifrontal form of the same factorization, where it has one
+            const MfPlan m = buildMfPlan(plan, s.nodeCol);
+            const std::string mf = m.node.empty() ? "" : checkMfPlan(plan, s.nodeCol, m);
             if (!mf.empty()) ++*violations;
             if (first.empty()) first = mf;
         }
@@ -291,6 +292,24 @@ extern "C" int olfgpu_structure_subtrees(int64_t structure, int64_t* stats6) {
             stats6[4] = binPos;
             stats6[5] = nbd.factorFrom;
         }
+    });
+}
+
+extern "C" int olfgpu_structure_multifrontal(int64_t structure, int64_t* stats5) {
+    return guarded([&] {
+        if (!stats5) throw std::runtime_error("null output");
+        const Structure& s = structureOf(structure)->host;
+        const MfPlan m = runsMultifrontal(s.plan) ? buildMfPlan(s.plan, s.nodeCol) : MfPlan{};
+        int front = 0, below = 0;
+        for (const MfNode& n : m.node) {
+            front = std::max(front, n.p + n.q);
+            below = std::max(below, n.q);
+        }
+        stats5[0] = static_cast<int64_t>(m.node.size());
+        stats5[1] = m.node.empty() ? 0 : static_cast<int64_t>(m.upPtr.size()) - 1;
+        stats5[2] = m.updBlocks;
+        stats5[3] = front;
+        stats5[4] = below;
     });
 }
 
@@ -458,6 +477,13 @@ extern "C" int olfgpu_set_schedule(int64_t context, int schedule, int lanesPerTi
         }
         c.schedule = schedule;
         c.autotunePending = false;
+    });
+}
+
+extern "C" int olfgpu_multifrontal_in_force(int64_t context, int* inForce) {
+    return guarded([&] {
+        if (!inForce) throw std::runtime_error("null output");
+        *inForce = contextOf(context).multifrontal() ? 1 : 0;
     });
 }
 

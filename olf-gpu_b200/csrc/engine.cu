@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <future>
 #include <numeric>
 
 namespace olfb200 {
@@ -420,6 +421,10 @@ std::shared_ptr<DeviceNet> uploadNet(const Structure& s) {
     OLF_CUDA(cudaGetDevice(&d->device));
     const BlockPlan& p = s.plan;
     const int nb = s.nb;
+    // the multifrontal plan (5 ms on 9,241 buses) is made beside the rest, on a thread of its own where one can be had
+    std::future<MfPlan> mf;
+    if (runsMultifrontal(p))
+        mf = std::async(std::launch::async | std::launch::deferred, [&] { return buildMfPlan(p, s.nodeCol); });
     auto aBlock = [&](int i, int j) {
         auto b = p.aCol.begin() + p.aPtr[i], e = p.aCol.begin() + p.aPtr[i + 1];
         auto it = std::lower_bound(b, e, j);
@@ -719,8 +724,8 @@ std::shared_ptr<DeviceNet> uploadNet(const Structure& s) {
     d->fwdSplitD.upload(d->fwdSplit);
     d->bwdSplitD.upload(d->bwdSplit);
     buildSubtreeBins(*d, p, lrowLen, splitOf);
-    if (!p.deferredL && nb >= MF_MIN_BUSES) {
-        d->mf = buildMfPlan(p, s.nodeCol);
+    if (mf.valid()) d->mf = mf.get();
+    if (!d->mf.node.empty()) {
         std::vector<MfNode> up, down;
         std::vector<MfTask> task;
         d->mfTaskPtr.assign(1, 0);
@@ -808,13 +813,11 @@ std::shared_ptr<const MfSchedules> DeviceNet::mfSchedules(int nS, int share) con
     auto s = std::make_shared<MfSchedules>();
     s->nS = nS;
     s->share = share;
-    if (!mf.node.empty()) {
-        const int S = (nS + 31) / 32 * 32;
-        s->up64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, true);
-        s->up32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, true);
-        s->down64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, false);
-        s->down32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, false);
-    }
+    const int S = (nS + 31) / 32 * 32;
+    s->up64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, true);
+    s->up32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, true);
+    s->down64 = scheduleMf(mf, mfTaskPtr, nS, S, share, false, false);
+    s->down32 = scheduleMf(mf, mfTaskPtr, nS, S, share, true, false);
     if (mfKept.size() >= 8) mfKept.erase(mfKept.begin());
     mfKept.push_back(s);
     return s;
@@ -1227,10 +1230,10 @@ void prepareMultifrontal(BatchContext& ctx, int share) {
     if (ctx.mfState == 2 || !ctx.regionFactor || !ctx.regionSolve || ctx.subtrees) return;
     if (ctx.mfState == 1 && ctx.mfSchedules->share == share) return;
     const DeviceNet& d = *ctx.dn;
+    if (d.mf.node.empty()) return;
     const auto schedules = d.mfSchedules(ctx.nS, share);
     if (ctx.mfState == 0) {
         ctx.mfState = 2;
-        if (!schedules->fits()) return;
         // one buffer for both precisions: a context's FP32 and FP64 factorizations never overlap
         const size_t bytes = static_cast<size_t>(std::max(d.mf.updBlocks, 1)) * 4 * ctx.S * 8;
         const ErrorMark mark;      // (the installs' launches before it are checked at the end of the solve)

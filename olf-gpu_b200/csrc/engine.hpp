@@ -84,7 +84,7 @@ struct DeviceNet {
     std::vector<int> topLevelPtr, topLevelSplit, topFwdPtr, topFwdSplit, topBwdPtr, topBwdSplit, binPhasePtr,
         binFwdPhasePtr, binBwdPhasePtr;
     int binTasks = 0;               // LU blocks the bins factorize (of nLu)
-    // the multifrontal plan (no nodes: a deferred-L plan or a small grid) and its device tables
+    // the multifrontal plan (no nodes: a deferred-L plan, a small grid or an order with a wide column) and its device tables
     MfPlan mf;
     std::vector<int> mfTaskPtr;      // the leaf levels' warp tasks
     // the launches of a batch of nS lanes: planned on first use, the last few sizes kept
@@ -237,8 +237,8 @@ struct BatchContext {
     bool regionSolve = false;       // level schedule: the solves' narrow levels in shared memory too
     bool subtrees = false;          // level schedule: the wide levels' independent subtrees as bins (schedule 5)
     // schedule 4's linear solve: the multifrontal plan's launches for this batch and its update matrices.  Made on first
-    // use (prepareMultifrontal); mfState 2: a small grid, a panel that fits no CTA or no room on the device for the update
-    // matrices, and the level launches with their narrow levels in shared memory run instead
+    // use (prepareMultifrontal).  Without a plan, or with no room on the device for the update matrices (mfState 2), the level
+    // launches with their narrow levels in shared memory run instead
     int mfState = 0;
     std::shared_ptr<const MfSchedules> mfSchedules;
     MfRun mfRun;

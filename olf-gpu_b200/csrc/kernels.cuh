@@ -341,14 +341,13 @@ struct MfSchedule {
 struct MfSchedules {
     int nS = 0, share = 1;
     MfSchedule up64, up32, down64, down32;
-    bool fits() const { return !up64.levels.empty() && !up32.levels.empty() && !down64.levels.empty() && !down32.levels.empty(); }
 };
 struct MfRun {
     MfDev dev{};
     const MfSchedule *up64 = nullptr, *up32 = nullptr, *down64 = nullptr, *down32 = nullptr;
     void* upd = nullptr;                                    // update matrices of every lane
 };
-// The launches of a batch of nS lanes (S with the padding) that runs beside share - 1 others; empty: some panel does not fit a CTA.
+// The launches of a batch of nS lanes (S with the padding) that runs beside share - 1 others.
 MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int nS, int S, int share, bool fp32, bool factor);
 cudaError_t prepareMf();
 // Factorization and forward solve of -F (w holds y, the U blocks their storage; FP32 also the L blocks), and the backward

@@ -658,7 +658,7 @@ __device__ __forceinline__ void factorNode(const DevBatch& b, T* lu, T* w, size_
 }
 
 // Strands a pivot row's columns below the pivots are split into (partial sums added in strand order).
-__host__ __device__ __forceinline__ int backwardStrands(int q) { return q <= 4 ? 1 : q <= 8 ? 2 : q <= 16 ? 4 : 8; }
+__host__ __device__ constexpr int backwardStrands(int q) { return q <= 4 ? 1 : q <= 8 ? 2 : q <= 16 ? 4 : 8; }
 
 // The backward substitution of one node, G lane pairs, one CTA: the rows below its pivots are solved.  Their columns first
 // (every pivot row and strand at once), then the pivot block is swept from its last row up.  sm: the pivot block [p][p], x
@@ -854,11 +854,20 @@ void launchLevels(const DevBatch& b, T* lu, T* wv, T* upd, const MfDev& mf, cons
     }
 }
 
-int teamBytes(const MfNode& n, int G, int elem, bool factor) {
-    const int m = n.p + n.q, bs = G * 2 * elem >= 128 ? 4 : 5;
-    if (factor) return ((n.p * (m + n.q) + n.p) * bs + n.p * 3) * G * 2 * elem;
-    return (n.p * n.p * bs + m * 2 + backwardStrands(n.q) * n.p * 2) * G * 2 * elem;
+constexpr int teamBytes(int p, int q, int G, int elem, bool factor) {
+    const int m = p + q, bs = G * 2 * elem >= 128 ? 4 : 5;
+    if (factor) return ((p * (m + q) + p) * bs + p * 3) * G * 2 * elem;
+    return (p * p * bs + m * 2 + backwardStrands(q) * p * 2) * G * 2 * elem;
 }
+int teamBytes(const MfNode& n, int G, int elem, bool factor) { return teamBytes(n.p, n.q, G, elem, factor); }
+
+// A plan's largest fronts (MF_MAX_PIVOTS pivots of MF_MAX_FRONT rows; one pivot over MF_MAX_BELOW) fit a CTA at one lane pair,
+// and their block numbers stay in smallDiv's range.
+constexpr bool frontFits(int p, int q) {
+    return teamBytes(p, q, 1, 8, true) <= MF_MAX_BYTES && teamBytes(p, q, 1, 8, false) <= MF_MAX_BYTES &&
+           p * (p + 2 * q) * (p + q) < 65536 && q * q * q < 65536;
+}
+static_assert(frontFits(MF_MAX_PIVOTS, MF_MAX_FRONT - MF_MAX_PIVOTS) && frontFits(1, MF_MAX_BELOW), "front limits");
 
 }  // namespace
 
@@ -924,8 +933,6 @@ MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int n
             // (never more pairs than the smaller panels before it: one segment per count)
             const int G = pairs(n, lv.segments ? std::min(cap, lv.seg[lv.segments - 1].pairs) : cap);
             const int bytes = teamBytes(n, G, elem, factor);
-            // a panel no CTA holds, or blocks past smallDiv's range: the caller keeps its level launches
-            if (bytes > MF_MAX_BYTES || n.p * (n.p + 2 * n.q) * (n.p + n.q) >= 65536 || n.q * n.q * n.q >= 65536) return MfSchedule{};
             MfSegment* sg = lv.segments ? &lv.seg[lv.segments - 1] : nullptr;
             if (!sg || sg->pairs != G) {
                 sg = &lv.seg[lv.segments++];

@@ -75,6 +75,12 @@ inline bool mfSmall(const MfNode& n) { return n.p == 1 && n.q <= 8; }
 // grid alone, so that a scenario's bits do not depend on its batch.
 constexpr int MF_MIN_BUSES = 512;
 constexpr int MF_MAX_PIVOTS = 16, MF_MAX_FRONT = 40, MF_LEAF_LEVELS = 5, MF_WARP_ROWS = 3;
+// The most rows below a pivot: the kernels divide a node's block numbers by multiplying with a 16-bit reciprocal.  An order
+// with a wider column gets no plan (no nodes), and its factorization keeps the level launches.
+constexpr int MF_MAX_BELOW = 40;
+
+// Plans that may run it (buildMfPlan may still find a column too wide).
+inline bool runsMultifrontal(const BlockPlan& p) { return !p.deferredL && p.nb >= MF_MIN_BUSES; }
 
 MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol);
 // "" when the plan holds: every position a pivot once, every LU block stored once, every Jacobian block and every

@@ -2,33 +2,113 @@
 #include "multifrontal.hpp"
 
 #include <algorithm>
-#include <map>
-#include <stdexcept>
+#include <cstdint>
+#include <utility>
 
 namespace olfb200 {
 
 namespace {
 
-// Appends one contribution to a target's (s0, s1) pair; a third and later one goes to `extra` (target -> list).
-struct Sources {
-    int s0 = -1, s1 = -1;
-    std::vector<int> extra;
-    void add(int s) {
-        if (s0 < 0) s0 = s;
-        else if (s1 < 0 && extra.empty()) s1 = s;
-        else extra.push_back(s);
+// What the targets of one node add up: the first two contributions of each, the others chained in their order of arrival.
+class Sources {
+public:
+    void reset(int targets) {
+        slot.assign(targets, Slot{});
+        extra.clear();
     }
+    void add(int target, int s) {
+        Slot& t = slot[target];
+        if (t.s0 < 0) {
+            t.s0 = s;
+        } else if (t.s1 < 0) {
+            t.s1 = s;
+        } else {
+            const int e = static_cast<int>(extra.size());
+            extra.push_back({s, -1});
+            if (t.first < 0) t.first = e;
+            else extra[t.last].next = e;
+            t.last = e;
+            t.more++;
+        }
+    }
+    // A target's (s0, s1); a third and later contribution goes to `more`.
+    void finish(int target, std::vector<int>& more, int& s0, int& s1) const {
+        const Slot& t = slot[target];
+        s0 = t.s0;
+        s1 = t.s1;
+        if (t.more == 0) return;
+        s1 = -2 - static_cast<int>(more.size());
+        more.push_back(t.more + 1);
+        more.push_back(t.s1);
+        for (int e = t.first; e >= 0; e = extra[e].next) more.push_back(extra[e].s);
+    }
+
+private:
+    struct Slot {
+        int s0 = -1, s1 = -1, first = -1, last = -1, more = 0;
+    };
+    struct Extra {
+        int s, next;
+    };
+    std::vector<Slot> slot;
+    std::vector<Extra> extra;
 };
 
-void finish(const Sources& s, std::vector<int>& more, int& s0, int& s1) {
-    s0 = s.s0;
-    s1 = s.s1;
-    if (s.extra.empty()) return;
-    s1 = -2 - static_cast<int>(more.size());
-    more.push_back(static_cast<int>(s.extra.size()) + 1);
-    more.push_back(s.s1);
-    more.insert(more.end(), s.extra.begin(), s.extra.end());
-}
+// First fit over a buffer that grows at its end: the free stretches by start in a tree of their largest lengths, so that the
+// lowest one that is long enough is found in a few steps.
+class FirstFit {
+public:
+    explicit FirstFit(int most) {
+        while (leaves < most) leaves *= 2;
+        longest.assign(2 * static_cast<size_t>(leaves), 0);
+        endOf.assign(most + 1, -1);
+    }
+    int take(int len) {
+        if (longest[1] < len) {
+            const int start = end;
+            end += len;
+            return start;
+        }
+        int x = 1;
+        while (x < leaves) x = longest[2 * x] >= len ? 2 * x : 2 * x + 1;
+        const int start = x - leaves, have = longest[x];
+        set(start, 0);
+        if (have > len) set(start + len, have - len);
+        return start;
+    }
+    void give(int start, int len) {
+        if (endOf[start] >= 0) {          // the stretch that ends here
+            const int before = endOf[start];
+            len += start - before;
+            set(before, 0);
+            start = before;
+        }
+        const int after = longest[leaves + start + len];
+        if (after > 0) {
+            set(start + len, 0);
+            len += after;
+        }
+        set(start, len);
+    }
+    int size() const { return end; }
+
+private:
+    int leaves = 1, end = 0;
+    std::vector<int> longest;      // [1]: of all; [leaves + start]: of the stretch starting there
+    std::vector<int> endOf;        // position -> start of the free stretch that ends there
+    void set(int start, int len) {
+        const int old = longest[leaves + start];
+        if (old > 0) endOf[start + old] = -1;
+        if (len > 0) endOf[start + len] = start;
+        int x = leaves + start;
+        longest[x] = len;
+        for (x /= 2; x >= 1; x /= 2) {
+            const int most = std::max(longest[2 * x], longest[2 * x + 1]);
+            if (longest[x] == most) break;
+            longest[x] = most;
+        }
+    }
+};
 
 }  // namespace
 
@@ -37,9 +117,12 @@ void finish(const Sources& s, std::vector<int>& more, int& s0, int& s1) {
 // pattern) are at most a third of the front.  A merge saves the column's update matrix (written and read back) and often
 // a tree level, and pays for the zeros in the panel.  Columns near the leaves (fewer than MF_LEAF_LEVELS levels of the
 // elimination tree below them) stay alone: there are thousands of them, and the one-pivot kernel is the cheaper one.
+// A column with more than MF_MAX_BELOW rows below its pivot: no plan (such a column would be a node of its own).
 MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol) {
     MfPlan r;
     const int nb = p.nb;
+    for (int k = 0; k < nb; k++)
+        if (p.uPtr[k + 1] - p.uPtr[k] - 1 > MF_MAX_BELOW) return r;
     std::vector<int> parentCol(nb, -1), rep(nb, -1), piv(nb, 0), below(nb, 0), height(nb, 0);
     for (int k = 0; k < nb; k++)
         if (p.uPtr[k + 1] - p.uPtr[k] > 1) {
@@ -101,16 +184,16 @@ MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol) {
     }
     auto byLevel = [&](const std::vector<int>& lev, bool smallFirst, std::vector<int>& ptr, std::vector<int>& order) {
         const int nl = nn ? 1 + *std::max_element(lev.begin(), lev.end()) : 0;
+        // by level, (small nodes first,) panel size, number
+        std::vector<std::pair<uint64_t, int>> key(nn);
+        for (int t = 0; t < nn; t++) {
+            const MfNode& n = r.node[t];
+            const uint64_t large = smallFirst && !mfSmall(n) ? 1 : 0;
+            key[t] = {(static_cast<uint64_t>(lev[t]) << 32) | (large << 31) | static_cast<uint64_t>(n.p * (n.p + 2 * n.q)), t};
+        }
+        std::sort(key.begin(), key.end());
         order.resize(nn);
-        for (int t = 0; t < nn; t++) order[t] = t;
-        auto panel = [&](int t) { return r.node[t].p * (r.node[t].p + 2 * r.node[t].q); };
-        std::sort(order.begin(), order.end(), [&](int a, int b) {
-            if (lev[a] != lev[b]) return lev[a] < lev[b];
-            const bool sa = mfSmall(r.node[a]), sb = mfSmall(r.node[b]);
-            if (smallFirst && sa != sb) return sa;
-            const int pa = panel(a), pb = panel(b);
-            return pa != pb ? pa < pb : a < b;
-        });
+        for (int t = 0; t < nn; t++) order[t] = key[t].second;
         ptr.assign(nl + 1, 0);
         for (int t = 0; t < nn; t++) ptr[lev[t] + 1]++;
         for (int l = 0; l < nl; l++) ptr[l + 1] += ptr[l];
@@ -124,69 +207,44 @@ MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol) {
     }
     // update matrices: first fit; a slot is free again one level after the parent's (whose launch reads it)
     {
-        std::map<int, int> freeAt;      // start -> length
-        int end = 0;
-        auto release = [&](int start, int len) {
-            auto nx = freeAt.lower_bound(start);
-            if (nx != freeAt.begin()) {
-                auto pv = std::prev(nx);
-                if (pv->first + pv->second == start) {
-                    start = pv->first;
-                    len += pv->second;
-                    freeAt.erase(pv);
-                }
-            }
-            if (nx != freeAt.end() && start + len == nx->first) {
-                len += nx->second;
-                freeAt.erase(nx);
-            }
-            freeAt[start] = len;
-        };
         auto size = [&](int t) { return r.node[t].q * r.node[t].q + (r.node[t].q + 1) / 2; };
+        int all = 0;
+        for (int t = 0; t < nn; t++) all += size(t);
+        FirstFit slots(all + 1);
         for (size_t l = 0; l + 1 < r.upPtr.size(); l++) {
             for (int x = r.upPtr[l]; x < r.upPtr[l + 1]; x++) {
-                const int t = r.upNode[x], len = size(t);
-                if (len == 0) continue;
-                auto it = freeAt.begin();
-                while (it != freeAt.end() && it->second < len) ++it;
-                if (it == freeAt.end()) {
-                    r.node[t].upd = end;
-                    end += len;
-                } else {
-                    const int start = it->first, have = it->second;
-                    freeAt.erase(it);
-                    r.node[t].upd = start;
-                    if (have > len) freeAt[start + len] = have - len;
-                }
+                const int t = r.upNode[x];
+                if (size(t) > 0) r.node[t].upd = slots.take(size(t));
             }
             for (int x = r.upPtr[l]; x < r.upPtr[l + 1]; x++)
                 for (int c : children[r.upNode[x]])
-                    if (size(c) > 0) release(r.node[c].upd, size(c));
+                    if (size(c) > 0) slots.give(r.node[c].upd, size(c));
         }
-        r.updBlocks = end;
+        r.updBlocks = slots.size();
     }
     // assembly: what each panel block, trailing block and right-hand-side row adds up
     r.pan.resize(nPan);
     r.trl.resize(nTrl);
     r.rhs.resize(nRows);
     std::vector<int> at(nb, -1);        // position -> front row of the node at hand
-    std::vector<Sources> front, rhs;
+    Sources front, rhs;
+    std::vector<int> out;
     for (int t = 0; t < nn; t++) {
         const MfNode& n = r.node[t];
         const int m = n.p + n.q;
         const int* rows = &r.rows[n.rows];
         for (int i = 0; i < m; i++) at[rows[i]] = i;
-        front.assign(static_cast<size_t>(m) * m, Sources{});
-        rhs.assign(m, Sources{});
+        front.reset(m * m);
+        rhs.reset(m);
         for (int c : children[t]) {
             const MfNode& k = r.node[c];
             const int* crow = &r.rows[k.rows + k.p];
             for (int a = 0; a < k.q; a++) {
-                for (int b = 0; b < k.q; b++) front[at[crow[a]] * m + at[crow[b]]].add(k.upd + a * k.q + b);
-                rhs[at[crow[a]]].add((k.upd + k.q * k.q) * 2 + a);
+                for (int b = 0; b < k.q; b++) front.add(at[crow[a]] * m + at[crow[b]], k.upd + a * k.q + b);
+                rhs.add(at[crow[a]], (k.upd + k.q * k.q) * 2 + a);
             }
         }
-        std::vector<int> out(static_cast<size_t>(m) * m, -1);
+        out.assign(static_cast<size_t>(m) * m, -1);
         for (int k = 0; k < n.p; k++) {
             const int pos = rows[k], u0 = p.uPtr[pos];
             out[k * m + k] = u0;
@@ -200,7 +258,7 @@ MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol) {
             MfPanel& e = r.pan[n.pan + idx];
             e.out = out[i * m + j];
             e.aBlock = e.out >= 0 ? p.luToA[e.out] : -1;
-            finish(front[i * m + j], r.more, e.s0, e.s1);
+            front.finish(i * m + j, r.more, e.s0, e.s1);
         };
         for (int k = 0; k < n.p; k++)
             for (int j = 0; j < m; j++) panel(k * m + j, k, j);
@@ -209,13 +267,13 @@ MfPlan buildMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol) {
         for (int a = 0; a < n.q; a++)
             for (int b = 0; b < n.q; b++) {
                 MfTrail& e = r.trl[n.trl + a * n.q + b];
-                finish(front[(n.p + a) * m + n.p + b], r.more, e.s0, e.s1);
+                front.finish((n.p + a) * m + n.p + b, r.more, e.s0, e.s1);
             }
         for (int i = 0; i < m; i++) {
             MfRhs& e = r.rhs[n.rows + i];
             e.rowP = i < n.p ? nodeCol[2 * p.perm[rows[i]]] : -1;
             e.rowV = i < n.p ? nodeCol[2 * p.perm[rows[i]] + 1] : -1;
-            finish(rhs[i], r.more, e.s0, e.s1);
+            rhs.finish(i, r.more, e.s0, e.s1);
         }
         for (int i = 0; i < m; i++) at[rows[i]] = -1;
     }
@@ -227,6 +285,14 @@ std::string checkMfPlan(const BlockPlan& p, const std::vector<int>& nodeCol, con
     auto fail = [](const std::string& what, int i) { return "multifrontal: " + what + " " + std::to_string(i); };
     std::vector<int> pivotOf(nb, -1), stored(nLu, 0), upLevel(nn, -1), downLevel(nn, -1);
     std::vector<char> aSeen(p.aCol.size(), 0);
+    // the shapes that the kernels' index arithmetic and shared memory are laid out for
+    for (int t = 0; t < nn; t++) {
+        const MfNode& n = m.node[t];
+        if (n.p < 1 || n.p > MF_MAX_PIVOTS || n.q > MF_MAX_BELOW || (n.p > 1 && n.p + n.q > MF_MAX_FRONT)) return fail("shape of node", t);
+    }
+    for (size_t l = 0; l < MF_LEAF_LEVELS && l + 1 < m.upPtr.size(); l++)
+        for (int x = m.upPtr[l]; x < m.upPtr[l + 1]; x++)
+            if (m.node[m.upNode[x]].p != 1) return fail("several pivots near the leaves, node", m.upNode[x]);
     for (int t = 0; t < nn; t++)
         for (int k = 0; k < m.node[t].p; k++) {
             const int pos = m.rows[m.node[t].rows + k];

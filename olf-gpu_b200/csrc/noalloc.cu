@@ -181,10 +181,10 @@ void linearSolveNoAlloc(const std::shared_ptr<NetStructure>& net, int nScenarios
     // launches instead of 122), the level launches otherwise.  FP32 keeps the level launches: its rounding follows the
     // summation order, and its results are those of the allocating entry point.
     std::shared_ptr<const MfSchedules> mf;
-    if (!fp32 && lay.withUpd <= NOALLOC_SCRATCH_BYTES) mf = dn.mfSchedules(nScenarios, 1);
+    if (!fp32 && !dn.mf.node.empty() && lay.withUpd <= NOALLOC_SCRATCH_BYTES) mf = dn.mfSchedules(nScenarios, 1);
     Hybrid hy{};
     MfRun run;
-    if (mf && mf->fits()) {
+    if (mf) {
         run = dn.mfRun(*mf, base + lay.upd);
         hy.mf = &run;
     }

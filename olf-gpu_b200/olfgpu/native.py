@@ -47,7 +47,8 @@ EXPORTS = ["olfgpu_last_error", "olfgpu_create_structure", "olfgpu_destroy_struc
            "olfgpu_linear_solve_transposed", "olfgpu_screen_violations", "olfgpu_last_slack_distribution_failures",
            "olfgpu_set_start_polish", "olfgpu_set_mixed_precision_policy", "olfgpu_last_fp64_iterations",
            "olfgpu_set_device_loop", "olfgpu_read_batch_targets", "olfgpu_read_batch_row_modes",
-           "olfgpu_structure_check_plan", "olfgpu_read_reactive_limits_state"]
+           "olfgpu_structure_check_plan", "olfgpu_read_reactive_limits_state", "olfgpu_structure_multifrontal",
+           "olfgpu_multifrontal_in_force"]
 # The arrays of BatchSolveNative.solveBatchContext this engine rejects when non-empty, in the reference's order
 UNSUPPORTED_SOLVE_ARRAYS = [
     "distributedSlackOverrideBus", "distributedSlackOverrideFactorDelta", "distributedSlackOverrideBaseTargetPDelta",
@@ -123,6 +124,8 @@ def load(path: str = LIB_PATH):
     L.olfgpu_set_device_loop.argtypes = [_i64, _ci]
     L.olfgpu_last_fp64_iterations.argtypes = [_i64, _ip]
     L.olfgpu_structure_subtrees.argtypes = [_i64, ctypes.POINTER(_i64)]
+    L.olfgpu_structure_multifrontal.argtypes = [_i64, ctypes.POINTER(_i64)]
+    L.olfgpu_multifrontal_in_force.argtypes = [_i64, _ip]
     L.olfgpu_linear_solve_transposed.argtypes = [_i64, _dp, _dp, _dp, _ci, _dp, _dp]
     L.olfgpu_screen_violations.argtypes = [_i64, _ci, _ip, _ip, _ip, _ip, _ip, _dp, _ci, _ip, _dp, _dp, _ci, _cd, _cd,
                                            _cd, _ci, _ip, _ip]
@@ -256,6 +259,12 @@ class Structure:
         _check(load().olfgpu_structure_check_plan(self.handle, planted_fault, ctypes.byref(v), msg, 512))
         return int(v.value), msg.value.decode()
 
+    def multifrontal(self) -> dict:
+        """The multifrontal plan of the block LU (zeros: the structure has none)."""
+        st = (_i64 * 5)()
+        _check(load().olfgpu_structure_multifrontal(self.handle, st))
+        return dict(nodes=st[0], levels=st[1], update_blocks=st[2], front_rows=st[3], rows_below=st[4])
+
     def recommend_batch_size(self, max_cap: int, mode: int = BATCHED_LU) -> int:
         b = ctypes.c_int(0)
         _check(load().olfgpu_recommend_batch_size(self.handle, max_cap, mode, ctypes.byref(b)))
@@ -345,6 +354,12 @@ class BatchContext:
                                           _p(res), ctypes.byref(nr)))
         tuning = [tuple(res[4 * i:4 * i + 4]) for i in range(min(nr.value, 32))]
         return (sc.value, la.value, th.value), tuning
+
+    def multifrontal_in_force(self) -> bool:
+        """Whether schedule 4 runs the multifrontal solve in this context (False before its first solve)."""
+        v = ctypes.c_int(0)
+        _check(load().olfgpu_multifrontal_in_force(self.handle, ctypes.byref(v)))
+        return bool(v.value)
 
     def solve(self, x0_base, target_base, base_row_mode, disabled, x0_full=None, row_mode_entries=None,
               target_override_index=None, target_override_value=None, max_iter: int = 15, tol: float = 1e-8,

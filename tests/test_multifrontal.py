@@ -30,6 +30,23 @@ def test_plan_holds(engine_lib, name, ordering):
     assert violations == 0, first
 
 
+@pytest.mark.parametrize("name,ordering,blocks", [
+    ("grid300", 19, 0), ("grid600", 19, None), ("grid600", 2, 0), ("grid2000", 19, 8356), ("grid2000", 1, 0),
+    ("grid2000", 8, 0), ("grid9241", 19, 41424), ("grid9241", 0, 36715), ("grid9241", 1, 0), ("grid13659", 0, 0)])
+def test_which_structures_have_a_plan(engine_lib, name, ordering, blocks):
+    """No plan for a small grid, a deferred-L plan and an order with more than 40 rows below some pivot: 104 in the natural
+    order of 600 buses, 52 and 128 by nested dissection, 44 by minimum degree on 13,659.  The update matrices' blocks a
+    lane are the memory a context takes."""
+    from olfgpu import native
+    p = (grid600() if name == "grid600" else grid(name))[1]
+    s = native.Structure(p, ordering)
+    mf = s.multifrontal()
+    assert (mf["nodes"] > 0) == (blocks != 0)
+    assert blocks is None or mf["update_blocks"] == blocks
+    assert mf["rows_below"] <= 40 and mf["front_rows"] <= 41
+    assert s.check_plan()[0] == 0
+
+
 # Both schedules solve the same 2x2 block systems in another summation order: a step's relative difference is about
 # eps * cond(J), 2e-16 * 1e5, and the iterations contract it; 1e-10 leaves a factor of five.
 STATE_TOL = 1e-10
