@@ -132,7 +132,8 @@ int olfgpu_structure_multifrontal(int64_t structure, int64_t* stats5);
 int olfgpu_structure_check_plan(int64_t structure, int plantedFault, int64_t* violations, char* firstViolation,
                                 int capacity);
 
-/* StructureNative.recommendBatchSize (structure_jni.cu:151-180): the bank that fits 70 % of free device memory. */
+/* StructureNative.recommendBatchSize (structure_jni.cu:151-180): the bank that fits 70 % of free device memory
+ * (schedule 4's update matrices included, where the structure has a multifrontal plan). */
 int olfgpu_recommend_batch_size(int64_t structure, int maxCap, int mode, int* batchOut);
 
 /*

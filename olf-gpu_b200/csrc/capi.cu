@@ -316,15 +316,30 @@ extern "C" int olfgpu_structure_multifrontal(int64_t structure, int64_t* stats5)
 extern "C" int olfgpu_recommend_batch_size(int64_t structure, int maxCap, int mode, int* batchOut) {
     return guarded([&] {
         if (!batchOut) throw std::runtime_error("null output");
-        const Structure& s = structureOf(structure)->host;
+        const std::shared_ptr<NetStructure> net = structureOf(structure);
+        const Structure& s = net->host;
         const BlockPlan& p = s.plan;
-        // what one lane of a context takes: state vectors, the Jacobian, the factors in the mode's precision
+        // what one lane of a context takes: state vectors, the Jacobian, the factors in the mode's precision, and the update
+        // matrices of the multifrontal solve
         const double lu = static_cast<double>(p.nU + p.nL) * 4 * (mode == MODE_BATCHED_LU ? 8 + 4 : 8);
-        const double perLane = 8.0 * s.n * 7 + s.n + static_cast<double>(p.aCol.size()) * 32 + lu + 8.0 * s.nb * 2 * 3;
+        const double rest = 8.0 * s.n * 7 + s.n + static_cast<double>(p.aCol.size()) * 32 + lu + 8.0 * s.nb * 2 * 3;
         size_t freeB = 0, totalB = 0;
         OLF_CUDA(cudaMemGetInfo(&freeB, &totalB));
         const double budget = 0.7 * static_cast<double>(freeB);
-        long fit = perLane > 0 ? static_cast<long>(budget / perLane) : maxCap;
+        auto fits = [&](double updates) { return static_cast<long>(budget / std::max(rest + updates * 32, 1.0)); };
+        // no node's slot is ever reused: an upper bound that needs no plan, and is enough away from the device's limit
+        double most = 0;
+        for (int k = 0; k < p.nb && runsMultifrontal(p); k++) {
+            const double d = p.uPtr[k + 1] - p.uPtr[k] - 1;
+            most += d * d + (d + 1) / 2;
+        }
+        long fit = fits(most);
+        if (fit < maxCap && most > 0) {
+            int device = 0;
+            OLF_CUDA(cudaGetDevice(&device));
+            const std::shared_ptr<DeviceNet> dn = net->find(device);
+            fit = fits(dn ? dn->mf.updBlocks : buildMfPlan(p, s.nodeCol).updBlocks);
+        }
         *batchOut = static_cast<int>(std::max<long>(1, std::min<long>(maxCap, fit)));
     });
 }

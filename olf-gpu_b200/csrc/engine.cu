@@ -1237,6 +1237,16 @@ void prepareMultifrontal(BatchContext& ctx, int share) {
         // one buffer for both precisions: a context's FP32 and FP64 factorizations never overlap
         const size_t bytes = static_cast<size_t>(std::max(d.mf.updBlocks, 1)) * 4 * ctx.S * 8;
         const ErrorMark mark;      // (the installs' launches before it are checked at the end of the solve)
+        // the level launches do without it, but not without what the context allocates later: the FP64 factors of a mixed
+        // batch (its first redo), the per-scenario starts
+        size_t later = ctx.full.p ? 0 : static_cast<size_t>(ctx.nS) * ctx.net->host.n * 8;
+        if (!ctx.lu64.p) later += static_cast<size_t>(d.view.nLu) * 4 * ctx.S * 8;
+        size_t freeBytes = 0, total = 0;
+        if (cudaMemGetInfo(&freeBytes, &total) != cudaSuccess) {
+            mark.drop();
+            return;
+        }
+        if (freeBytes < bytes + later + (size_t(64) << 20)) return;      // (64 MiB: the graphs, the runtime's own)
         if (cudaMalloc(&ctx.mfUpd.p, bytes) != cudaSuccess) {
             mark.drop();
             ctx.mfUpd.p = nullptr;
@@ -1729,6 +1739,14 @@ cudaGraphConditionalHandle newHandle(cudaGraph_t owner) {
     return h;
 }
 
+// What a device-resident Newton loop cannot do without.
+void allocLoop(BatchContext& ctx) {
+    const size_t blocks = static_cast<size_t>(ctx.dn->view.nLu) * 4 * ctx.S;
+    if (ctx.precision == 1 && !ctx.lu32.p) ctx.lu32.alloc(blocks * 4);
+    if (!ctx.lu64.p) ctx.lu64.alloc(blocks * 8);
+    if (!ctx.loopState.p) ctx.loopState.alloc(8 * sizeof(int));
+}
+
 // Appends one context's device-resident Newton loop to graph g as a branch with no dependencies: the loop state reset,
 // the WHILE node, the cap of lanes still iterating, and (withResults) the scenario-major result gather.  Three
 // capture streams: cs[0] for the branch, cs[1] for the WHILE body, cs[2] for the bodies nested in it.
@@ -1737,10 +1755,7 @@ void appendNewtonLoop(BatchContext& ctx, cudaGraph_t g, const cudaStream_t* cs, 
     const DeviceNet& dn = *ctx.dn;
     const DevNet& net = dn.view;
     const bool mixed = ctx.precision == 1;
-    const size_t S = ctx.S;
-    if (mixed && !ctx.lu32.p) ctx.lu32.alloc(static_cast<size_t>(net.nLu) * 4 * S * 4);
-    if (!ctx.lu64.p) ctx.lu64.alloc(static_cast<size_t>(net.nLu) * 4 * S * 8);
-    if (!ctx.loopState.p) ctx.loopState.alloc(8 * sizeof(int));
+    allocLoop(ctx);
     prepareMultifrontal(ctx, share);
     const DevBatch b = ctx.batch();
     const DevBatch b64 = fp64View(ctx), b64all = fp64AllView(ctx);
@@ -2260,6 +2275,7 @@ void launchMultiLoops(MultiContext& m) {
         if (!m.capStreams[0]) {
             for (auto& s : m.capStreams) OLF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         }
+        for (BatchContext* c : m.members) allocLoop(*c);      // before any member's update matrices, which are optional
         cudaGraph_t g;
         OLF_CUDA(cudaGraphCreate(&g, 0));
         m.loopKeys.clear();

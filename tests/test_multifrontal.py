@@ -88,3 +88,75 @@ def test_a_lane_does_not_depend_on_its_batch(engine_lib):
         rows[count] = ctx.solve(p.x_base, p.target, p.base_row_mode, p.outage_masks(outs[:count]))[0].copy()
     for count, row in rows.items():
         assert np.array_equal(row, rows[150]), count
+
+
+def _leave_free(nbytes):
+    """A device array that leaves about nbytes of the memory free."""
+    import torch
+    torch.cuda.empty_cache()
+    return torch.empty(torch.cuda.mem_get_info()[0] - nbytes, dtype=torch.uint8, device="cuda")
+
+
+LANES, MARGIN = 2048, 300 << 20       # MARGIN: well under the update matrices of so many lanes (547 MB)
+
+
+@pytest.mark.gpu
+def test_no_room_for_the_update_matrices(engine_lib):
+    """The level launches run in their place, with their results; the context has room for nothing more than its factors."""
+    import torch
+    from olfgpu import native, synthetic
+    g, p = grid("grid2000")
+    dis = p.outage_masks(np.resize(synthetic.draw_outages(g, 64, seed=3), LANES))
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    res = []
+    for full in (False, True):
+        ctx = native.BatchContext(s, LANES)
+        ctx.set_schedule(native.LEVELS_SHARED_ALL, 0, 256)
+        filler = _leave_free(s.n_lu_blocks * 32 * LANES + MARGIN) if full else None
+        res.append(ctx.solve(p.x_base, p.target, p.base_row_mode, dis))
+        assert ctx.multifrontal_in_force() != full
+        del filler, ctx
+        torch.cuda.empty_cache()
+    a, b = res
+    conv = a[:, -1] == 0
+    assert np.array_equal(a[:, -1], b[:, -1]) and np.max(np.abs(a[conv, :p.n] - b[conv, :p.n])) < STATE_TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("device_loop", [False, True])
+def test_update_matrices_leave_room_for_the_fp64_redo(engine_lib, device_loop):
+    """A mixed batch with room for its FP32 and FP64 factors, which it allocates on the first redo, and for little more."""
+    import torch
+    from olfgpu import native, synthetic
+    g, p = grid("grid2000")
+    dis = p.outage_masks(np.resize(synthetic.draw_outages(g, 64, seed=3), LANES))
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    ctx = native.BatchContext(s, LANES)
+    ctx.set_schedule(native.LEVELS_SHARED_ALL, 0, 256)
+    ctx.set_linear_solver_settings(native.MIXED, 3)
+    ctx.set_mixed_precision_controls(1e-2, 1.0)      # every pivot is over the limit: every lane is factorized again in FP64
+    ctx.set_device_loop(device_loop)
+    filler = _leave_free(s.n_lu_blocks * 48 * LANES + MARGIN)
+    out = ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
+    assert ctx.last_fp64_refactors().size == LANES and not ctx.multifrontal_in_force()
+    assert (out[:, -1] == 0).any()
+    del filler, ctx
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,ordering", [("grid2000", 19), ("grid2000", 1), ("grid118", 19)])
+def test_recommended_batch_counts_the_update_matrices(engine_lib, name, ordering):
+    import torch
+    from olfgpu import native
+    _, p = grid(name)
+    s = native.Structure(p, ordering)
+    lane = 8 * p.n * 7 + p.n + s.n_a_blocks * 32 + s.n_lu_blocks * 48 + 8 * p.n * 3
+    lane += s.multifrontal()["update_blocks"] * 32
+    free = torch.cuda.mem_get_info()[0]
+    got = s.recommend_batch_size(1 << 30)
+    native.BatchContext(s, 1)
+    again = s.recommend_batch_size(1 << 30)        # the plan on the device is asked, where there is one
+    for v in (got, again):
+        assert abs(v * lane / (0.7 * free) - 1) < 2e-2
+    assert s.recommend_batch_size(8) == 8
