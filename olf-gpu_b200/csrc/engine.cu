@@ -1874,14 +1874,19 @@ int runDeviceLoop(BatchContext& ctx) {
     return ctx.hostActive[5];
 }
 
+// The factors of the context's precision and the multifrontal solve's launches and memory, made on first use.
+void prepareFactors(BatchContext& ctx) {
+    const size_t blocks = static_cast<size_t>(ctx.dn->view.nLu) * 4 * ctx.S;
+    if (ctx.precision == 1 && !ctx.lu32.p) ctx.lu32.alloc(blocks * 4);
+    if (ctx.precision != 1 && !ctx.lu64.p) ctx.lu64.alloc(blocks * 8);
+    prepareMultifrontal(ctx, 1);
+}
+
 int runIterations(BatchContext& ctx) {
     cudaStream_t st = ctx.stream;
     const DeviceNet& dn = *ctx.dn;
     const bool mixed = ctx.precision == 1;
-    const size_t S = ctx.S;
-    if (mixed && !ctx.lu32.p) ctx.lu32.alloc(static_cast<size_t>(dn.view.nLu) * 4 * S * 4);
-    if (!mixed && !ctx.lu64.p) ctx.lu64.alloc(static_cast<size_t>(dn.view.nLu) * 4 * S * 8);
-    prepareMultifrontal(ctx, 1);
+    prepareFactors(ctx);
     const int cap = roundCap(ctx);
     if (ctx.fallbackStart && ctx.hasX0Base && ctx.hasX0Full) selectStarts(ctx);
     if (ctx.deviceLoop && !ctx.phaseTiming && ctx.schedule != SCHEDULE_PERSISTENT && ctx.schedule != SCHEDULE_COOP) {
@@ -2002,6 +2007,7 @@ void autotune(BatchContext& ctx) {
     };
     for (const Candidate& c : cands) {
         apply(c);
+        prepareFactors(ctx);      // not part of what is timed
         installLanes(ctx);
         OLF_CUDA(cudaEventRecord(e0, ctx.stream));
         runIterations(ctx);
@@ -2361,6 +2367,9 @@ void autotuneMulti(MultiContext& m, bool fp32) {
     m.tuning.clear();
     bool tilesFit = true;      // the persistent tiles run neither dense-front plans nor the extra outer loops / tests
     for (const BatchContext* c : m.members) tilesFit = tilesFit && multiTilesFit(*c);
+    // not part of what is timed: the members' factors and the multifrontal solve's launches and memory
+    for (BatchContext* c : m.members) allocLoop(*c);
+    for (BatchContext* c : m.members) prepareMultifrontal(*c, static_cast<int>(m.members.size()));
     {
         m.lanesPerTile = 0;
         OLF_CUDA(cudaEventRecord(e0, m.stream));
