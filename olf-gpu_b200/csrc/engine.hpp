@@ -30,23 +30,31 @@ struct DeviceBuffer {
     ~DeviceBuffer() {
         if (p) cudaFree(p);
     }
+    // The zero fill is complete on return: the contexts' streams do not wait for the default stream it runs on.
     void alloc(size_t n) {
-        if (p) cudaFree(p);
-        p = nullptr;
-        bytes = n;
+        reserve(n);
         if (n) {
-            OLF_CUDA(cudaMalloc(&p, n));
             OLF_CUDA(cudaMemset(p, 0, n));
+            OLF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
         }
     }
     template <typename T>
     void upload(const std::vector<T>& v) {
-        alloc(v.size() * sizeof(T));
+        reserve(v.size() * sizeof(T));
         if (!v.empty()) OLF_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
     }
     template <typename T>
     T* as() const {
         return static_cast<T*>(p);
+    }
+
+private:
+    void reserve(size_t n) {
+        if (p) cudaFree(p);
+        p = nullptr;
+        bytes = 0;
+        if (n) OLF_CUDA(cudaMalloc(&p, n));
+        bytes = n;
     }
 };
 

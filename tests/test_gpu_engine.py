@@ -592,3 +592,24 @@ def test_config1_every_non_bridge_outage_of_the_2000_bus_grid(engine_lib, oracle
     ref = oracle_mod.Structure(p).solve_batch(p.x_base, dis)
     _compare(r, ref, p.n)
     assert np.array_equal(r[:, p.n].astype(int), ref[:, p.n].astype(int))
+
+
+@pytest.mark.parametrize("schedule,threads", [(0, 256), (2, 512), (4, 256)])
+def test_fp64_redo_on_its_first_use(engine_lib, schedule, threads):
+    """Mixed precision with every lane over the pivot-growth limit: the first iteration of a new context allocates the FP64
+    factors in mid-solve and is the FP64 context's iteration (the same matrices; the mismatch after one step at rounding)."""
+    from olfgpu import native, synthetic
+    g, p = grid("grid2000")
+    dis = p.outage_masks(synthetic.draw_outages(g, 150, seed=21))
+    s = native.Structure(p)
+    ref = native.BatchContext(s, 150)
+    want = ref.solve(p.x_base, p.target, p.base_row_mode, dis, max_iter=1)
+    for _ in range(4):
+        ctx = native.BatchContext(s, 150)
+        ctx.set_linear_solver_settings(native.MIXED, 0)
+        ctx.set_mixed_precision_controls(1e-2, 1.0)
+        ctx.set_fp64_restart(False)
+        ctx.set_schedule(schedule, 0, threads)
+        got = ctx.solve(p.x_base, p.target, p.base_row_mode, dis, max_iter=1)
+        assert ctx.last_fp64_refactors().size == 150
+        assert np.max(np.abs(got[:, :p.n] - want[:, :p.n])) < 1e-9
