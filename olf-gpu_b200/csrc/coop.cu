@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(512) factorCoopKernel(DevNet net, DevBatch b, 
     const int gtid = (blockIdx.x * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
     for (int s = gtid; s < b.S; s += nthreads)
         if (coopSolving(b, s)) b.trouble[s] = 0;
+    grid.sync();      // before any CTA's first level flags a pivot
     const int vy = b.S / 32;
     for (int l = 0; l < cp.nLevels; l++) {
         const int first = cp.levelPtr[l], count = cp.levelPtr[l + 1] - first;
