@@ -113,7 +113,7 @@ int olfgpu_structure_subtrees(int64_t structure, int64_t* stats6);
 /*
  * The multifrontal plan of the structure's block LU (no counterpart in the reference; schedule 4 of olfgpu_set_schedule
  * and the FP64 no-allocation solve run it): {nodes, levels of the assembly tree, 2x2 blocks of one lane's update matrices,
- * rows of the largest front, most rows below a node's pivots} into stats5.  Zeros: no plan, for a grid under 512 buses, a
+ * rows of the largest front, most rows below a node's pivots} into stats5.  Zeros: no plan, for a grid under 700 buses, a
  * deferred-L plan, or an elimination order in which some pivot has more than 40 rows below it.
  */
 int olfgpu_structure_multifrontal(int64_t structure, int64_t* stats5);

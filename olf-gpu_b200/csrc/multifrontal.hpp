@@ -69,11 +69,14 @@ inline bool mfSmall(const MfNode& n) { return n.p == 1 && n.q <= 8; }
 // to MF_WARP_ROWS rows below the pivot; one row of it otherwise: four rows' blocks spill); further up a CTA does.
 // Factorization + solves per pass, 9,241 buses, 500 / 17 lanes, by leaf levels: 3 2.26 / 0.74 ms, 5 2.14 / 0.68 ms,
 // 7 2.13 / 0.68 ms, 9 2.09 / 0.69 ms; 2,000 buses, 257 lanes: 0.31, 0.33, 0.35, 0.36 ms.
-// Grids from here on take the multifrontal solve; below, the few levels of the level launches are the shorter chain (whole
-// solves, device time: 118 buses, 130 lanes 0.72 ms against 0.85 ms, 300 buses, 130 lanes 0.83 against 0.94, 1 lane 0.80
-// against 0.87; 2,000 buses, 1 / 16 / 257 lanes 0.84 / 1.19 / 2.55 ms against 0.62 / 0.84 / 2.03 ms).  The line depends on the
-// grid alone, so that a scenario's bits do not depend on its batch.
-constexpr int MF_MIN_BUSES = 512;
+// Grids from here on take the multifrontal solve; below, the few levels of the level launches are the shorter chain.  Whole
+// solves, level launches / multifrontal, ms, 1 and 130 lanes: 512 buses 0.74 / 0.77 and 3.32 / 3.55, 540 0.74 / 0.83 and 3.35 /
+// 3.77, 640 0.55 / 0.57 and 3.35 / 3.47, 660 (three grids, all batch sizes) 0.5 to 11 % slower; 700 (three grids) 0.95 / 0.81
+// and 4.47 / 3.45, 0.94 / 0.85 and 4.53 / 3.81, 0.79 / 0.80 and 1.38 / 1.33; 820 0.96 / 0.90 and 4.41 / 4.01; 1,000 1.32 / 1.11
+// and 5.09 / 4.39; 2,000 1.28 / 0.97 and 2.28 / 1.80; 9,241 3.29 / 2.07 and 7.09 / 5.30.  Small mixed batches gain as well (8
+// lanes: 2,000 buses 3.43 / 2.79, 9,241 5.45 / 3.96).  The line is one of the grid, not of the batch: a scenario's bits do not
+// depend on its batch's size, on any batch that has room for the update matrices.
+constexpr int MF_MIN_BUSES = 700;
 constexpr int MF_MAX_PIVOTS = 16, MF_MAX_FRONT = 40, MF_LEAF_LEVELS = 5, MF_WARP_ROWS = 3;
 // The most rows below a pivot: the kernels divide a node's block numbers by multiplying with a 16-bit reciprocal.  An order
 // with a wider column gets no plan (no nodes), and its factorization keeps the level launches.
