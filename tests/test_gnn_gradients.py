@@ -98,3 +98,41 @@ def test_message_gradients_match(engine_lib, B):
     bound = gd.n_edges * 2.0 ** -24
     assert float((we - ref).abs().max()) <= bound * float((gd.es.abs().T @ dc32.abs()).max())
     assert float((db[0] - refb).abs().max()) <= bound * float(dc32.abs().sum(0).max())
+
+
+@pytest.mark.parametrize("B", [1, 3, 9])
+def test_message_gradients_match_float64(engine_lib, B):
+    """dPQ and dC of both entries against sums over the edges in float64, the outaged branch's edges left out.  The inputs are
+    such that no pre-activation is near zero (a ReLU's side does not hang on rounding): FP32 sums of as many terms as a bus has
+    edges or an edge has samples, 16 * 2^-24 of the terms' magnitudes; BF16, of eight significant bits, adds half a unit in the last, 2^-8 of the result."""
+    import torch
+    from olfgpu import gnn
+    g, _ = grid("grid118")
+    gd = gnn.GraphData.from_grid(g)
+    gen = torch.Generator(device="cuda").manual_seed(40 + B)
+    nb, M = gd.nb, B * gd.nb
+    # multiples of 1/4, and an odd multiple of 1/8 in the bias: exact in BF16 and FP32, and never a sum of zero
+    quarter = lambda *s: torch.randint(-8, 9, s, device="cuda", generator=gen).float() / 4  # noqa: E731
+    pq, C, bm = quarter(M, 128).to(torch.bfloat16), quarter(gd.n_edges, 64), quarter(64) + 0.125
+    dagg = torch.randn((M, 64), device="cuda", generator=gen)
+    outage = torch.arange(B, dtype=torch.int32, device="cuda") * 7
+    src, dst, branch = gd.src.long(), gd.dst.long(), gd.branch.long()
+    PQ, D = pq.double().reshape(B, nb, 128), dagg.double().reshape(B, nb, 64)
+    pre = PQ[:, src, :64] + PQ[:, dst, 64:] + C.double() + bm.double()
+    on = (pre > 0) & (branch[None, :] != outage.long()[:, None])[..., None]
+    ge = torch.where(on, D[:, dst], torch.zeros_like(pre))
+    want = torch.zeros((B, nb, 128), dtype=torch.float64, device="cuda")
+    want[:, :, :64].index_add_(1, src, ge)
+    want[:, :, 64:].index_add_(1, dst, ge)
+    size = torch.zeros_like(want)
+    size[:, :, :64].index_add_(1, src, ge.abs())
+    size[:, :, 64:].index_add_(1, dst, ge.abs())
+    want, size = want.reshape(M, 128), size.reshape(M, 128)
+    for name, dtype, ulp in (("olfgpu_gnn_message_backward", torch.float32, 0.0),
+                             ("olfgpu_gnn_message_backward_bf16", torch.bfloat16, 2.0 ** -8)):
+        out, dc = torch.full((M, 128), 7.0, dtype=dtype, device="cuda"), torch.full((gd.n_edges, 64), 7.0, device="cuda")
+        gnn._call(name, B, nb, gd.n_edges, *[gnn._ptr(t) for t in (gd.in_ptr, gd.in_edge, gd.out_ptr, gd.out_edge, gd.src,
+                  gd.dst, gd.branch, outage, pq, C, bm, dagg, out, dc)], gnn._stream())
+        bound = 16 * 2.0 ** -24 * size
+        assert bool(((out.double() - want).abs() <= bound + ulp * (want.abs() + bound)).all())
+        assert bool(((dc.double() - ge.sum(0)).abs() <= 16 * 2.0 ** -24 * ge.abs().sum(0)).all())

@@ -190,3 +190,86 @@ def test_autotuner_times_the_solve_without_its_preparation(engine_lib):
         ms.append(min(t[3] for t in ctx.schedule()[1] if t[0] == native.LEVELS_SHARED_ALL))
         assert ctx.schedule()[0][0] == native.LEVELS_SHARED_ALL
     assert ms[0] < 2 * ms[1]
+
+
+def _fp32_step(native, p, s, dis, schedule, steps):
+    """The state after one iteration of FP32 factors, refined in that many steps (0: not at all); no lane is redone."""
+    ctx = native.BatchContext(s, dis.shape[0])
+    ctx.set_linear_solver_settings(native.MIXED, steps)
+    ctx.set_mixed_precision_controls(1e30, 1e30)
+    ctx.set_fp64_restart(False)
+    ctx.set_schedule(*schedule)
+    out = ctx.solve(p.x_base, p.target, p.base_row_mode, dis, max_iter=1)
+    assert ctx.last_fp64_refactors().size == 0 and ctx.multifrontal_in_force() == (schedule[0] == 4)
+    return out[:, :p.n]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,ordering,count", [("grid760", 19, 1), ("grid760", 1, 3), ("grid760", 0, 66), ("grid2000", 19, 17),
+                                                 ("grid2000", 16, 130)])
+def test_fp32_factors_match_the_level_launches(engine_lib, name, ordering, count):
+    """FP32 factors in another summation order: a step from them is about as far from the FP64 step as the level launches' is
+    (four times as far at most).  Three refinement steps, which read the stored L blocks, contract both by FP32's error of the
+    solution (under 1e-2) each: what is left is FP64 rounding, 1e-10 as for the states."""
+    from olfgpu import native, synthetic
+    g, p = any_grid(name)
+    dis = p.outage_masks(synthetic.draw_outages(g, count, seed=11 + count))
+    s = native.Structure(p, ordering)
+    ctx = native.BatchContext(s, count)
+    want = ctx.solve(p.x_base, p.target, p.base_row_mode, dis, max_iter=1)[:, :p.n]
+    err = {sch: [np.abs(_fp32_step(native, p, s, dis, (sch, 0, 256), steps) - want).max() for steps in (0, 3)] for sch in (0, 4)}
+    assert 0 < err[4][0] <= 4 * err[0][0]
+    assert err[4][1] <= 1e-10 and err[0][1] <= 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [(5,), (8,), (6, 7)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_singular_lanes_fail_alone(engine_lib, bad, precision):
+    """An islanded PQ bus (its angle column is zero) in the odd lane of a pair, the even one, or both: the pivot is flagged
+    there at the first factorization, the others keep their bits."""
+    from olfgpu import native, synthetic
+    from test_status_rules import _islanding_mask, _pq_bus
+    g, p = grid("grid2000")
+    dis = p.outage_masks(synthetic.draw_outages(g, 13, seed=3))
+    broken = dis.copy()
+    broken[list(bad)] = _islanding_mask(p, g, _pq_bus(p, g))[0]
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    ctx = native.BatchContext(s, 13)
+    ctx.set_linear_solver_settings(precision, 3)
+    ctx.set_schedule(native.LEVELS_SHARED_ALL, 0, 256)
+    clean = ctx.solve(p.x_base, p.target, p.base_row_mode, dis).copy()
+    r = ctx.solve(p.x_base, p.target, p.base_row_mode, broken)
+    assert ctx.multifrontal_in_force()
+    keep = [k for k in range(13) if k not in bad]
+    assert np.all(r[list(bad), -1] == native.LINEAR_SOLVE_FAILED) and np.all(r[list(bad), p.n] == 0)
+    assert np.array_equal(r[keep], clean[keep])
+
+
+@pytest.mark.gpu
+def test_one_context_alone_and_among_others(engine_lib):
+    """A context solved alone, in a launch of several (its launches planned for its share of the GPU), and alone again, with
+    the device loop and without: the same bits each time, and the members' graph is still good afterwards."""
+    from olfgpu import native, synthetic
+    from olfgpu.security_analysis import ConcurrentBatch
+    g, p = grid("grid2000")
+    dis = p.outage_masks(synthetic.draw_outages(g, 90, seed=9))
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    cb = ConcurrentBatch(s, 90, 3)
+    (a, b), c = cb.ranges[1], cb.contexts[1]
+
+    def alone(device_loop):
+        c.set_device_loop(device_loop)
+        out = c.solve(p.x_base, p.target, p.base_row_mode, dis[a:b]).copy()
+        c.set_device_loop(True)
+        return out
+
+    rows = [alone(False), alone(True)]
+    among = [cb.solve(p.x_base, p.target, p.base_row_mode, dis)[0].copy()]
+    rows += [alone(True), alone(False)]
+    among.append(cb.solve(p.x_base, p.target, p.base_row_mode, dis)[0].copy())
+    assert all(x.multifrontal_in_force() for x in cb.contexts)
+    assert np.array_equal(among[0], among[1])
+    for r in rows:
+        assert np.array_equal(r, among[0][a:b])
+    cb.close()
