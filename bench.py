@@ -32,12 +32,15 @@ GRID = "grid9241"
 N_OUTAGES = 500
 TOL = 1e-8
 CHECKPOINT = os.path.join(ROOT, "olf-gpu_b200", "checkpoints", "warmstart_grid9241.npz")
-# DRAM bytes (read + write) of one lane's factorization (narrow levels in shared memory), from ncu captures of the
+# DRAM bytes (read + write) of one lane's factorization, from ncu captures of the launches of the first factorization of a
+# 64-outage batch: multifrontal on the shallow-tree order (21 launches, FP64 317.4 MB over 64 lanes); level launches with the
+# narrow levels in shared memory, from ncu captures of the
 # launches of the first factorization of a 64-outage batch: the dense-front plan on plain minimum degree (89 launches;
 # FP64 490.9 MB, FP32 LU 288.3 MB over 64 lanes) and on the shallow-tree order (123 launches; 573.2 MB, 328.6 MB);
 # scaled to a launch by the lanes it factorizes
 TRAFFIC = {("dense", "fp64"): 7.67e6, ("dense", "mixed"): 4.51e6,
            ("shallow", "fp64"): 8.96e6, ("shallow", "mixed"): 5.13e6}
+TRAFFIC_MULTIFRONTAL = {("shallow", "fp64"): 4.96e6}
 
 
 def _peaks():
@@ -137,11 +140,13 @@ NARROW, REGION_SLOTS, REGION_THREADS, SOLVE_REGION_SLOTS = 48, 110 * 1024 // 32,
 GNN_LAUNCHES = 1 + 4 * 4 + 1 + 1 + 2
 
 
-def launches_per_solve(s, sched, rounds: int, dense: bool, deferred: bool, mixed: bool, refine_rounds: int) -> int:
+def launches_per_solve(s, sched, rounds: int, dense: bool, deferred: bool, mixed: bool, refine_rounds: int,
+                       multifrontal: bool = False) -> int:
     """Kernels one batch solve launches: per factorizing round the factorization (level launches, the range or the
     shared-memory region, the dense front), the solves, step and advance; per round the start, fill, test and lane
-    count; per solve the install and result gathers (6).  Matches the ncu launch lists: 802 per FP64 solve of the
-    9,241-bus / 500-outage batch under schedule 4, 782 under the level schedule with 2-lane tiles (scaled plan)."""
+    count; per solve the install and result gathers (6).  Matches the ncu launch lists: per FP64 solve of the 9,241-bus /
+    500-outage batch 802 under schedule 4's level launches, 782 under the level schedule with 2-lane tiles (scaled plan);
+    with the multifrontal solve 206, and 3 more where the linear solve is scored (not counted)."""
     schedule, lanes = int(sched[0]), int(sched[1])
     f, _, fw, bw = s.levels()
     wf, wfw, wbw = np.diff(f), np.diff(fw), np.diff(bw)
@@ -168,6 +173,9 @@ def launches_per_solve(s, sched, rounds: int, dense: bool, deferred: bool, mixed
     front = 1 if dense else 0
     if schedule == 1:                       # the whole Newton loop in one persistent launch
         return 1 + 6
+    if schedule == 4 and multifrontal:      # a launch per level of the assembly tree; the forward solve rides along
+        levels = s.multifrontal()["levels"]
+        return int(rounds * (1 + levels + levels + 2 + (1 if mixed else 0)) + (rounds + 1) * 4 + 6 + refine_rounds * 3)
     if schedule == 2:                       # cooperative sweeps: one launch per factorization and per sweep
         factor, solve = 1 + 1 + front, 2 + front + 2
     else:
@@ -388,8 +396,8 @@ def run_engine(args, rank: int, world: int):
     refine_bytes = refinement if args.mixed_policy == "refine" else 0
     total_bytes, b_it = algorithmic_bytes(s, p, tot_iters // args.steps, pbytes, refine_bytes)
     achieved = total_bytes / (dev * 1e-3) / 1e9
-    # the dominant kernel family, the block-LU factorization (factorLevelKernel + factorRangeKernel launches of one
-    # Newton iteration): one more solve of the same batch, after the timed region, with each phase bracketed by CUDA
+    # the dominant kernel family, the block-LU factorization (the factorization launches of one Newton iteration; the
+    # multifrontal form's solve the forward system as well): one more solve of the same batch, after the timed region, with each phase bracketed by CUDA
     # events on the context's stream; algorithmic bytes of one lane's factorization = read J once (8 nnzJ) + write and
     # read the LU once (2 w nnzLU)
     ctx.set_phase_timing(True)
@@ -405,18 +413,22 @@ def run_engine(args, rank: int, world: int):
     fact_launch_ms = ph["factor"] / max(ph["iterations"], 1)
     fact_bytes_launch = fact_bytes_lane * ph["factorized_lanes"] / max(ph["iterations"], 1)
     fact_achieved = fact_bytes_launch / (fact_launch_ms * 1e-3) / 1e9 if fact_launch_ms > 0 else 0.0
-    traffic = TRAFFIC.get((args.plan, "fp64" if fact_w == 8 else "mixed"))
+    multifrontal = ctx.multifrontal_in_force()
+    traffic = (TRAFFIC_MULTIFRONTAL if multifrontal else TRAFFIC).get((args.plan, "fp64" if fact_w == 8 else "mixed"))
     if traffic is not None:
         traffic = int(traffic * ph["factorized_lanes"] / max(ph["iterations"], 1))
     sched = ctx.schedule()[0]
     fact_kernel = "block-LU factorization of one Newton iteration (factorLevelKernel levels"
-    if sched[0] in (native.LEVELS_SHARED, native.LEVELS_SHARED_ALL):
+    if multifrontal:
+        fact_kernel = ("block-LU factorization of one Newton iteration, forward solve included (mfLeafKernel / mfLevelKernel, a "
+                       "launch per level of the assembly tree")
+    elif sched[0] in (native.LEVELS_SHARED, native.LEVELS_SHARED_ALL):
         fact_kernel += " + regionPrefixKernel / regionFactorKernel narrow levels in shared memory"
     elif sched[0] == native.LEVELS and sched[1] > 0:
         fact_kernel += " + factorRangeKernel narrow levels"
     elif sched[0] == native.COOPERATIVE:
         fact_kernel = "block-LU factorization of one Newton iteration (factorCoopKernel"
-    fact_kernel += (" + denseFrontKernel)" if dense_front(args.plan) else ")")
+    fact_kernel += " + denseFrontKernel)" if dense_front(args.plan) and not multifrontal else ")"
     if ph["iterations"] == 0:
         # the autotuner picked the persistent schedule: one launch runs the whole Newton loop of the batch
         fact_kernel = "newtonPersistentKernel (the whole Newton loop of the batch in one launch)"
@@ -501,17 +513,27 @@ def run_engine(args, rank: int, world: int):
                       "solve_levels": s.forward_levels + s.backward_levels, "block_ops": s.block_ops},
         "clocks": sampler.summary(),
     }
-    rounds = max(ph["iterations"], 1)
-    per_solve = launches_per_solve(s, sched, rounds, dense_front(args.plan), args.plan == "deferred",
-                                   precision == native.MIXED and fp64_iterations < rounds,
-                                   (rounds - 1) if refinement > 0 and args.mixed_policy == "refine" else 0)
-    if args.device_loop:
-        per_solve += 2 + rounds * (2 if precision == native.MIXED else 1)   # loop reset, cap; a condition per round
+    # the measured solve: one context, or the concurrent parts, each a loop of its own over its factorizing rounds
+    if cb is None:
+        loops = [(sched, max(ph["iterations"], 1), multifrontal)]
+    else:
+        loops = [(part_schedule, max(int(c.last_stats()[1]) - 1, 1), c.multifrontal_in_force()) for c in cb.contexts]
+    per_solve = 0
+    for loop_sched, rounds, mf in loops:
+        per_solve += launches_per_solve(s, loop_sched, rounds, dense_front(args.plan), args.plan == "deferred",
+                                        precision == native.MIXED and fp64_iterations < rounds,
+                                        (rounds - 1) if refinement > 0 and args.mixed_policy == "refine" else 0, mf)
+        if args.device_loop:
+            per_solve += 2 + rounds * (2 if precision == native.MIXED else 1)   # loop reset, cap; a condition per round
+        if learned is not None:
+            per_solve += 6                     # the two-start selection (2 fills and 4 small kernels)
     if learned is not None:
-        per_solve += GNN_LAUNCHES + 6          # the prediction, the two-start selection (2 fills and 4 small kernels)
+        per_solve += GNN_LAUNCHES              # the prediction
     line["gpu_launches"] = int(per_solve * args.steps)
     line["gpu_launches_basis"] = (f"{per_solve} per step: the level structure under the schedule in force over "
-                                  f"{rounds} factorizing Newton rounds (the same count as the ncu launch lists)")
+                                  f"{[r for _, r, _ in loops]} factorizing Newton rounds, "
+                                  f"{'multifrontal' if all(m for _, _, m in loops) else 'level'} linear solve "
+                                  "(counted as the ncu launch lists do)")
     if not args.no_uneven:
         line["uneven_batch"] = uneven_summary(args)
     if rank == 0 and not args.no_cpu_baseline:
@@ -695,7 +717,7 @@ def run_uneven(args, rank: int, world: int):
         launches = 0
         for (st, c, p, dis), r in zip(seq, rounds):
             launches += launches_per_solve(st, member, max(r, 1), dense_front(args.plan), args.plan == "deferred",
-                                           precision == native.MIXED, 0) + 2 + max(r, 1)
+                                           precision == native.MIXED, 0, st.multifrontal()["nodes"] > 0) + 2 + max(r, 1)
     else:
         launches = 1 + 4 + 5 * 4
     line = {

@@ -28,6 +28,14 @@ def test_launch_count_matches_the_launch_lists(bench_mod):
     assert bench_mod.launches_per_solve(dense, (4, 0, 256), 4, True, False, False, 0) == 802
 
 
+def test_launch_count_of_the_multifrontal_solve(bench_mod):
+    from olfgpu import native
+    _, p, _ = bench_mod.workload(0, 500)
+    s = native.Structure(p, native.PLAN_DEFAULT)
+    # 1,045 launches over five solves, less the three of each solve's scoring
+    assert bench_mod.launches_per_solve(s, (4, 0, 256), 4, True, False, False, 0, True) == 1045 // 5 - 3
+
+
 def test_reference_arm_prints_the_contract_line(tmp_path):
     """`bench.py --impl reference` (the oracle on the host cores, a bounded sample of the same outages) prints one JSON
     line with the engine arm's metric and unit, its own cpu_baseline and an e2e object with no device copies."""
