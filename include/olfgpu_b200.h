@@ -585,7 +585,9 @@ int olfgpu_gnn_compose_start_compact(int nScenarios, int nb, const float* predBa
  * first call after the device's CUDA context was re-created (cudaDeviceReset); make that first call before any stream
  * capture.  All calls share the one array and it keeps the previous call's contents (what must start at zero is
  * cleared on every call): calls whose work overlaps on the GPU race, so order them on one stream.  A scenario whose
- * factorization meets a (near-)singular 2x2 pivot gets NaN in every entry of its outDevice row.
+ * factorization meets a (near-)singular 2x2 pivot gets NaN in every entry of its outDevice row.  FP64 batches of a
+ * structure with a multifrontal plan (olfgpu_structure_multifrontal) run it where its update matrices fit the array beside
+ * the rest, and the level launches otherwise: between batches of those two sizes a solution may differ by rounding.
  */
 int olfgpu_linear_solve_noalloc(int64_t structure, int nScenarios, const double* csrValsDevice,
                                 const double* rhsDevice, double* outDevice, int precision, void* stream);

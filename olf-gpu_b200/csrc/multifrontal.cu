@@ -16,8 +16,9 @@
 // (pair g, worker).  A level with few nodes takes few pairs and many workers per pair (latency), one with many nodes small
 // CTAs (their fixed latencies overlap).  Every sum has an order that does not depend on G or on the CTA's size.
 //
-// What bounds it: near the leaves memory (9,241 buses, 500 lanes: the first level moves 0.87 GB in 0.19 ms, 4.6 TB/s),
-// further up the dependent loads and FP64 latencies of a node (15 to 60 us a level; the FP64 pipe is under 10 % busy).
+// What bounds it: near the leaves memory (9,241 buses, 500 lanes: the first level reads and writes 0.93 GB in 0.19 ms, 5.0
+// TB/s, the four after it 3.8 to 4.2 TB/s), further up the dependent loads and FP64 latencies of a node (64 lanes: 23 to 48 us a
+// level; the FP64 pipe is 4 to 6 % busy, near the leaves under 10 %).
 // Factorization + solves of one pass on 9,241 buses, 500 / 17 lanes: 2.68 / 1.12 ms with the level launches, 2.14 / 0.68 ms
 // here; two lanes a thread took the 500-lane pass from 2.90 to 2.40 ms.
 //
@@ -873,6 +874,7 @@ static_assert(frontFits(MF_MAX_PIVOTS, MF_MAX_FRONT - MF_MAX_PIVOTS) && frontFit
 
 MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int nS, int S, int share, bool fp32,
                       bool factor) {
+    constexpr int SMS = 148;      // B200's; only the launches' shapes follow it, no result does
     MfSchedule r;
     const std::vector<int>& ptr = factor ? plan.upPtr : plan.downPtr;
     const std::vector<int>& order = factor ? plan.upNode : plan.downNode;
@@ -923,8 +925,8 @@ MfSchedule scheduleMf(const MfPlan& plan, const std::vector<int>& taskPtr, int n
         const MfNode* largest = firstTeam < ptr[l + 1] ? &plan.node[order[ptr[l + 1] - 1]] : nullptr;
         for (lv.threads = WIDE_CTA;; lv.threads /= 2) {
             for (cap = 1; cap < top && cap < nP;) cap *= 2;
-            while (cap > 1 && ctas() < 148 / share) cap /= 2;
-            if (lv.threads == 32 || ctas() * lv.threads <= 148L * 512 / share) break;
+            while (cap > 1 && ctas() < SMS / share) cap /= 2;
+            if (lv.threads == 32 || ctas() * lv.threads <= SMS * 512L / share) break;
             // (the largest panel, at whole sectors, would take more than the narrower CTAs' share)
             if (lv.threads <= CTA && largest && teamBytes(*largest, std::min(cap, whole), elem, factor) > MF_SHARE_BYTES * (lv.threads / 2) / CTA) break;
         }

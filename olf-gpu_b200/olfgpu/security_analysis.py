@@ -191,7 +191,7 @@ class ConcurrentBatch:
     structure, solved by ONE graph launch whose branches are the parts' device-resident Newton loops (the engine's
     multi-grid context with lanesPerTile 0).  The parts' level kernels run concurrently, so one part's dependent-level
     latency overlaps another's work.  Every scenario's result is that of the single batch, bit for bit (lanes never
-    interact).  ``solve`` takes the arguments of BatchContext.stage for the whole batch."""
+    interact), unless the device has room for some contexts' multifrontal update matrices and not for others'.  ``solve`` takes the arguments of BatchContext.stage for the whole batch."""
 
     def __init__(self, structure: native.Structure, n_scenarios: int, parts: int, precision: int = native.FP64,
                  refinement_steps: int = 1, mixed_policy: int = native.MIXED_REFINE,
