@@ -175,20 +175,19 @@ def test_recommended_batch_counts_the_update_matrices(engine_lib, name, ordering
 
 @pytest.mark.gpu
 def test_autotuner_times_the_solve_without_its_preparation(engine_lib):
-    """A new context's first tuning gives schedule 4 about the time of a second one: its planning and allocation took three
-    times the solve.  The best of four contexts, since a shared host holds single solves up."""
+    """A new context's first tuning gives schedule 4 about the time of a second one: its planning and allocation came on
+    top.  The best of four networks, since a shared host holds single solves up."""
     from olfgpu import native, synthetic
     g, p = grid("grid9241")
     dis = p.outage_masks(synthetic.draw_outages(g, 17, seed=3))
-    s = native.Structure(p, native.PLAN_DEFAULT)
     ms = np.full((4, 2), np.inf)
     for k in range(4):
-        ctx = native.BatchContext(s, 17)
+        ctx = native.BatchContext(native.Structure(p, native.PLAN_DEFAULT), 17)
         for again in range(2):
             ctx.set_schedule(-1, 0, 0)
             ctx.solve(p.x_base, p.target, p.base_row_mode, dis)
             ms[k, again] = min(t[3] for t in ctx.schedule()[1] if t[0] == native.LEVELS_SHARED_ALL)
-    assert ms[:, 0].min() < 2 * ms[:, 1].min()
+    assert ms[:, 0].min() < 1.1 * ms[:, 1].min(), ms      # 1.18 to 3.5 with the preparation, 0.99 to 1.01 without
 
 
 def _fp32_step(native, p, s, dis, schedule, steps):
